@@ -325,7 +325,8 @@ def _matrices(case, seed):
     n, count = case["n"], case["count"]
     g = torch.Generator(device="cuda").manual_seed(seed)
     if case["matrix"] == "orthogonal":
-        return torch.linalg.qr(torch.randn(count, n, n, generator=g, dtype=F64, device="cuda"))[0]
+        q = torch.linalg.qr(torch.randn(count, n, n, generator=g, dtype=F64, device="cuda"))[0]
+        return q.contiguous()
     scale = torch.logspace(0, 2, n, dtype=F64, device="cuda")
     out = torch.empty(count, n, n, dtype=F64, device="cuda")
     for a, b in _chunks(count, 60 * n):
