@@ -201,18 +201,15 @@ int me_plan_tail_slots(const me_plan *plan);
  * Results agree with one thread per pixel to rounding. */
 int me_plan_max_group(const me_plan *plan);
 void me_plan_set_max_group(me_plan *plan, int lanes);
-/* Lanes per 9x9 SVD in the LM rounds that still feed from the queue (1, 2, 4
- * or 8); more lanes cut the decomposition's latency, fewer keep more of them
- * in flight.  Default 1. */
+/* Lanes per SVD in the LM rounds that still feed from the queue (1, 2, 4 or 8)
+ * when a parameter is fixed; more lanes cut the decomposition's latency, fewer
+ * keep more of them in flight.  Default 1.  With all nine free one thread
+ * serves a matrix; any value above 1 then only selects the lane groups'
+ * rounding. */
 int me_plan_svd_lanes(const me_plan *plan);
-/* With all nine parameters free, the SVD solves can keep their 9x9 matrix in
- * registers, one thread per pixel: 0 (default) = shared memory everywhere;
- * 1 = registers in the one-thread-per-pixel rounds; 2 = registers also in the
- * lane-split rounds after the queue drains (in place of the lanes' shared
- * SVD).  Same operations in the same order (results agree to rounding: the
- * compiler fuses multiply-adds differently); the register form has no
- * shared-memory round trips, the shared-memory form a smaller code.  Which is
- * faster depends on the batch (me_plan_autotune tries them). */
+/* Kept for programs that set it (0, 1 or 2): with all nine parameters free the
+ * SVD solves hold their 9x9 matrix in registers, one thread per pixel, in every
+ * round, whatever this says. */
 int me_plan_svd_registers(const me_plan *plan);
 void me_plan_set_svd_registers(me_plan *plan, int mode);
 /* The LM rounds between two checks of the queue go to the GPU as one CUDA
@@ -324,8 +321,7 @@ int me_faddeeva_weideman(const double *nu, const double *a, long n, double *H, d
  * flight (window), lanes per pixel after the queue drains (max_group), the
  * tail kernel's threshold (tail_slots), lanes per SVD (svd_lanes), the
  * kernel variant (pixels per CTA, grid staging, Faddeeva series reciprocals;
- * me_plan_set_kernel_variant), where the SVD keeps its matrix
- * (me_plan_set_svd_registers), the lanes and check interval after the
+ * me_plan_set_kernel_variant), the lanes and check interval after the
  * queue drains (me_plan_set_drain), the FP32 Faddeeva evaluation
  * (me_plan_set_faddeeva) and the slot-major profile copy
  * (me_plan_set_slot_profiles) -- one knob at a time, keeping each

@@ -238,9 +238,7 @@ int build_devplan(const me_config *cfg, const double *lambda, int nl, DevPlan &P
     P.regul_weight[i] = cfg->regul_weight[i];
   }
   if (P.npar == 0) return fail(ME_ERR_CONFIG, "all nine parameters are fixed");
-  // measured defaults on a B200 (the autotuner may choose others): the
-  // shared-memory SVD; on the FP32 path the Jacobian kernel with its sums in
-  // shared memory
+  // measured defaults on a B200 (the autotuner may choose others)
   P.svd_regs = 0;
   P.kvar = 0;
   P.faddeeva = cfg->precision == ME_PREC_FP32 ? 1 : 0;
@@ -719,10 +717,10 @@ int run_queue(me_plan *p, const me::InvertArgs &A, cudaStream_t st, long long &r
   int grids[3];
   grids[0] = std::min(p->grid_jac, (W + me::kBlock - 1) / me::kBlock);
   grids[1] = std::min(p->grid_trial, (W + me::kBlock - 1) / me::kBlock);
-  grids[2] = p->svd_lanes > 1
+  grids[2] = p->svd_lanes > 1 && p->P.npar < 9
                  ? (int)std::min<long long>(p->grid_trial,
                                             ((long long)W * p->svd_lanes + me::kBlock - 1) / me::kBlock)
-                 : std::min(p->grid_svd, (W + me::kSvdBlock - 1) / me::kSvdBlock);
+                 : me::svd_grid(p->P.npar, p->grid_svd, W);
   int parity = 0;
   int group = 1;              // lanes per slot of the next rounds
   int ggrids[3] = {1, 1, 1};  // their grids
@@ -863,7 +861,8 @@ int run_queue(me_plan *p, const me::InvertArgs &A, cudaStream_t st, long long &r
       const long long need = ((long long)W * g + me::kBlock - 1) / me::kBlock;
       ggrids[0] = (int)std::min<long long>(p->grid_jac, need);
       ggrids[1] = (int)std::min<long long>(p->grid_trial, need);
-      ggrids[2] = (int)std::min<long long>(p->grid_trial, need);
+      ggrids[2] = p->P.npar == 9 ? me::svd_grid(9, p->grid_svd, W)
+                                 : (int)std::min<long long>(p->grid_trial, need);
     }
     // default: half a wave of the tail kernel's warps
     const int tail = p->tail_slots < 0 ? p->grid_fin * (me::kBlock / 32) / 2 : p->tail_slots;
@@ -1573,9 +1572,6 @@ extern "C" int me_plan_autotune(me_plan *p, const double *d_prof, long npix, voi
       // the wavelength grid staged in shared memory, no reciprocal table, the
       // normal-equation sums in shared memory
       {&p->P.kvar, {0, 1, 2, 3, 4, 5}},
-      // the 9x9 SVD in registers in the full rounds, also in the lane-split
-      // rounds, or in shared memory throughout (the default)
-      {&p->P.svd_regs, {1, 2, 0}},
       // after the queue drains: lanes per pixel in flight (half a wave to four
       // waves of the Jacobian kernel) and rounds between checks
       {&p->group_fill, {1, 2, 4, 8}},

@@ -495,7 +495,8 @@ __device__ __forceinline__ int solve_slot(const DevPlan &P, const Slots &S, int 
 }
 
 // solve_slot for a plan with all nine parameters free, one thread per slot,
-// the matrix in registers (gr_svd_u9): the same trial steps and ladder.
+// the matrix in registers (gr_svd9; FORM 0 gives the bits of solve_slot with
+// one thread, FORM 1 those of its lane groups): the same trial steps and ladder.
 // Trial 1 decomposes H; trial 2 uses the factor trial 1 stored; trial
 // k >= 3 decomposes the factor trial k - 1 left (see solve_slot).
 __device__ __forceinline__ void trial_params9(const DevPlan &P, const Slots &S, int s,
@@ -509,8 +510,9 @@ __device__ __forceinline__ void trial_params9(const DevPlan &P, const Slots &S, 
   store9(S.ptmp, W, s, ptmp);
 }
 
-template <bool FAST>
-__device__ __forceinline__ int solve_slot9(const DevPlan &P, const Slots &S, int s) {
+template <int FORM, bool FAST, int STR>
+__device__ __forceinline__ int solve_slot9(const DevPlan &P, const Slots &S, int s, double *w,
+                                           double *rv1, double *cs) {
   const int W = S.W;
   const int tk = S.tk[s];
   double x[9];
@@ -528,12 +530,12 @@ __device__ __forceinline__ int solve_slot9(const DevPlan &P, const Slots &S, int
     trial_params9(P, S, s, x);
     return 0;
   }
-  double A[9][9], w[9];
+  double A[9][9];
 #pragma unroll
   for (int r = 0; r < 9; r++)
 #pragma unroll
     for (int c = 0; c < 9; c++) A[r][c] = S.hess[(size_t)(r * 9 + c) * W + s];
-  const int hits = gr_svd_u9<FAST>(A, w);
+  const int hits = gr_svd9<FORM, FAST, STR>(A, w, rv1, cs);
 #pragma unroll
   for (int r = 0; r < 9; r++)
 #pragma unroll
@@ -554,17 +556,17 @@ __device__ __forceinline__ int solve_slot9(const DevPlan &P, const Slots &S, int
   if (tk == 1) {
     double wmax = w[0];
 #pragma unroll
-    for (int i = 1; i < 9; i++) wmax = fmax(wmax, w[i]);
+    for (int i = 1; i < 9; i++) wmax = fmax(wmax, w[i * STR]);
     double thr = P.svd_thr;
     while (true) {
       const double wthr = wmax * thr;
       double tj[9];
 #pragma unroll
       for (int j = 0; j < 9; j++) {
-        double wj = w[j];
+        double wj = w[j * STR];
         if (wj < wthr) {
           wj = 0.0;
-          w[j] = 0.0;
+          w[j * STR] = 0.0;
         }
         tj[j] = wj > 1e-50 ? ug[j] / wj : 0.0;
       }
@@ -832,21 +834,33 @@ static __global__ void __launch_bounds__(kSvdBlock) svd_kernel(const __grid_cons
   tl.flush(A, S);
 }
 
-// svd_kernel for plans with all nine parameters free: each thread's matrix in
-// its registers (solve_slot9), no shared memory.
-template <bool FAST>
+// The same for plans with all nine parameters free: each thread's matrix in its
+// registers (solve_slot9), w and rv1 in its columns of shared memory.  Each
+// warp takes `per` slots at a time, the fewest (a power of two) for which the
+// grid covers the list in one pass: a warp's time is that of the longest of
+// its matrices' sweeps, so few slots spread over all the warps.
+template <int FORM, bool FAST>
 static __global__ void __launch_bounds__(kSvdBlock) svd9_kernel(const __grid_constant__ DevPlan P,
                                                                 const __grid_constant__ InvertArgs A,
                                                                 const __grid_constant__ Slots S,
                                                                 int parity, int which) {
+  __shared__ double sm[kSvd9Words * kSvdBlock];
+  const int t = threadIdx.x, lane = t & 31;
+  double *w = sm + t, *rv1 = sm + 9 * kSvdBlock + t, *cs = sm + 18 * kSvdBlock + t;
   const int W = S.W;
   Tally tl;
   const int *list = which == 0 ? S.jlist + parity * W : S.rlist + parity * W;
   const int count = which == 0 ? S.jcount[parity] : S.rcount[parity];
-  for (int i = blockIdx.x * kSvdBlock + threadIdx.x; i < count; i += gridDim.x * kSvdBlock) {
-    const int s = list[i];
-    if (S.state[s] != SL_TRIAL) continue;
-    tl.svdlim += solve_slot9<FAST>(P, S, s);
+  const int warps = gridDim.x * (kSvdBlock / 32);
+  int per = 1;
+  while (per < 32 && warps * per < count) per *= 2;
+  if (lane < per) {
+    for (int i = (blockIdx.x * (kSvdBlock / 32) + t / 32) * per + lane; i < count;
+         i += warps * per) {
+      const int s = list[i];
+      if (S.state[s] != SL_TRIAL) continue;
+      tl.svdlim += solve_slot9<FORM, FAST, kSvdBlock>(P, S, s, w, rv1, cs);
+    }
   }
   tl.flush(A, S);
 }
@@ -1326,19 +1340,24 @@ int round_grid_impl(int which, int device) {
   } else if (which == 3) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, finish_kernel<T, FILT>, kBlock, 0);
   } else {
-    // the larger of the two SVD kernels' resident grids (a grid beyond one
-    // kernel's residency only queues blocks)
     cudaFuncSetAttribute(svd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSvdSmem);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, svd_kernel, kSvdBlock, kSvdSmem);
-    int per_sm9 = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm9, svd9_kernel<false>, kSvdBlock, 0);
-    int per_sm9f = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm9f, svd9_kernel<true>, kSvdBlock, 0);
-    if (per_sm9f > per_sm9) per_sm9 = per_sm9f;
-    if (per_sm9 > per_sm) per_sm = per_sm9;
+    // svd9_kernel's registers allow the same four CTAs of 64; a grid beyond
+    // one kernel's residency would only queue blocks
   }
   if (per_sm < 1) per_sm = 1;
   return sms * per_sm;
+}
+
+// The solves with all nine parameters free: `grid` CTAs, at most one resident
+// wave (round_grid(2), svd_grid).
+template <int FORM>
+static inline void launch_svd9(const DevPlan &P, const InvertArgs &A, const Slots &S, int parity,
+                               int which, int grid, cudaStream_t st) {
+  if (P.fastg)
+    svd9_kernel<FORM, true><<<grid, kSvdBlock, 0, st>>>(P, A, S, parity, which);
+  else
+    svd9_kernel<FORM, false><<<grid, kSvdBlock, 0, st>>>(P, A, S, parity, which);
 }
 
 // static: svd_kernel has internal linkage, so each translation unit must launch
@@ -1348,18 +1367,18 @@ int round_grid_impl(int which, int device) {
 static inline void launch_svd_lanes(int lanes, const DevPlan &P, const InvertArgs &A,
                                     const Slots &S, int parity, int which, int grid,
                                     cudaStream_t st) {
+  if (P.npar == 9) {
+    if (lanes > 1)
+      launch_svd9<1>(P, A, S, parity, which, grid, st);
+    else
+      launch_svd9<0>(P, A, S, parity, which, grid, st);
+    return;
+  }
   switch (lanes) {
     case 2: svd_grp_kernel<2><<<grid, kBlock, 0, st>>>(P, A, S, parity, which); break;
     case 4: svd_grp_kernel<4><<<grid, kBlock, 0, st>>>(P, A, S, parity, which); break;
     case 8: svd_grp_kernel<8><<<grid, kBlock, 0, st>>>(P, A, S, parity, which); break;
-    default:
-      if (P.npar == 9 && P.svd_regs && P.fastg)
-        svd9_kernel<true><<<grid, kSvdBlock, 0, st>>>(P, A, S, parity, which);
-      else if (P.npar == 9 && P.svd_regs)
-        svd9_kernel<false><<<grid, kSvdBlock, 0, st>>>(P, A, S, parity, which);
-      else
-        svd_kernel<<<grid, kSvdBlock, kSvdSmem, st>>>(P, A, S, parity, which);
-      break;
+    default: svd_kernel<<<grid, kSvdBlock, kSvdSmem, st>>>(P, A, S, parity, which); break;
   }
 }
 
@@ -1428,16 +1447,13 @@ cudaError_t launch_round_impl(const DevPlan &P, const InvertArgs &A, const Slots
 }
 
 // The SVD launches of a lane-split round: G lanes per matrix in shared memory
-// (svd_grp_kernel), or, with P.svd_regs == 2 and all nine parameters free,
-// one thread per matrix in registers (svd9_kernel; the grid of G-lane groups
-// has at least one thread per slot).
+// (svd_grp_kernel), or, with all nine parameters free, one thread per matrix in
+// registers (svd9_kernel).
 template <int G>
 static inline void launch_svd_grp(const DevPlan &P, const InvertArgs &A, const Slots &S,
                                   int parity, int which, int grid, cudaStream_t st) {
-  if (P.npar == 9 && P.svd_regs == 2 && P.fastg)
-    svd9_kernel<true><<<grid * (kBlock / kSvdBlock), kSvdBlock, 0, st>>>(P, A, S, parity, which);
-  else if (P.npar == 9 && P.svd_regs == 2)
-    svd9_kernel<false><<<grid * (kBlock / kSvdBlock), kSvdBlock, 0, st>>>(P, A, S, parity, which);
+  if (P.npar == 9)
+    launch_svd9<1>(P, A, S, parity, which, grid, st);
   else
     svd_grp_kernel<G><<<grid, kBlock, 0, st>>>(P, A, S, parity, which);
 }

@@ -29,6 +29,13 @@ constexpr int kSvdBlock = 64;  // threads of svd_kernel; each holds its matrix i
 constexpr int kKernelVariants = 6;
 constexpr int kMaxStage = 1024;
 constexpr int kSvdSmem = (81 + 18) * kSvdBlock * 8;
+// CTAs of the SVD launches with one thread per matrix over W slots: with all
+// nine parameters free (svd9_kernel) up to a warp per slot, else a thread
+inline int svd_grid(int npar, int wave, int W) {
+  const int per = npar == 9 ? kSvdBlock / 32 : kSvdBlock;
+  const int need = (W + per - 1) / per;
+  return need < wave ? need : wave;
+}
 // learned initialiser inference: rows per chunk, kernel launches per chunk
 constexpr int kMlpPredChunk = 65536;
 constexpr int kMlpPredLaunches = 6;

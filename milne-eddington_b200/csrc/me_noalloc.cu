@@ -261,9 +261,7 @@ extern "C" int me_invert_batch_device_noalloc(const me_config *cfg, const double
                                                              : (W + me::kBlock - 1) / me::kBlock;
   grids[1] = d->grids[1] < (W + me::kBlock - 1) / me::kBlock ? d->grids[1]
                                                              : (W + me::kBlock - 1) / me::kBlock;
-  grids[2] = d->grids[2] < (W + me::kSvdBlock - 1) / me::kSvdBlock
-                 ? d->grids[2]
-                 : (W + me::kSvdBlock - 1) / me::kSvdBlock;
+  grids[2] = me::svd_grid(P.npar, d->grids[2], W);
   rc = run_rounds(prec, P, A, S, grids, st, d_small);
   if (rc) return rc;
 

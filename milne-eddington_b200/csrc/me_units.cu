@@ -414,6 +414,50 @@ __global__ void __launch_bounds__(32) svd_u_kernel(const double *a, long long nm
   if (hit && limit_hits && (G == 1 || t % G == 0)) atomicAdd(limit_hits, 1);
 }
 
+// The decomposition of 9 x 9 matrices, one thread per matrix in registers
+// (gr_svd9), `per` matrices per warp: a warp's matrices come in and go out
+// through shared memory, so that global memory is read and written in whole
+// lines (stride 81: no bank conflict).
+template <int FORM, bool FAST>
+__global__ void __launch_bounds__(32) svd_u9_kernel(const double *a, long long nmat, int per,
+                                                    double *u, double *w, int *limit_hits) {
+  __shared__ double tile[32 * 81];
+  __shared__ double wr[kSvd9Words * 32];
+  const int t = threadIdx.x;
+  const long long first = blockIdx.x * (long long)per;
+  const int here = (int)(nmat - first < per ? nmat - first : per);
+  for (int k = t; k < here * 81; k += 32) tile[k] = a[first * 81 + k];
+  __syncwarp();
+  if (t < here) {
+    double A[9][9];
+#pragma unroll
+    for (int r = 0; r < 9; r++)
+#pragma unroll
+      for (int c = 0; c < 9; c++) A[r][c] = tile[t * 81 + r * 9 + c];
+    const int hit = gr_svd9<FORM, FAST, 32>(A, wr + t, wr + 9 * 32 + t, wr + 18 * 32 + t);
+#pragma unroll
+    for (int r = 0; r < 9; r++)
+#pragma unroll
+      for (int c = 0; c < 9; c++) tile[t * 81 + r * 9 + c] = A[r][c];
+    if (hit && limit_hits) atomicAdd(limit_hits, 1);
+  }
+  __syncwarp();
+  for (int k = t; k < here * 81; k += 32) u[first * 81 + k] = tile[k];
+  for (int k = t; k < here * 9; k += 32) w[first * 9 + k] = wr[(k % 9) * 32 + k / 9];
+}
+
+template <int FORM>
+static void launch_svd_u9(const double *d_a, long long nmat, int fast, double *d_u, double *d_w,
+                          int *d_hits, cudaStream_t st) {
+  int per = 32;
+  while (per > 1 && (nmat + per / 2 - 1) / (per / 2) <= 148 * 8) per /= 2;
+  const unsigned g = (unsigned)((nmat + per - 1) / per);
+  if (fast)
+    svd_u9_kernel<FORM, true><<<g, 32, 0, st>>>(d_a, nmat, per, d_u, d_w, d_hits);
+  else
+    svd_u9_kernel<FORM, false><<<g, 32, 0, st>>>(d_a, nmat, per, d_u, d_w, d_hits);
+}
+
 template <int G>
 static void launch_svd_u_g(const double *d_a, long long nmat, int n, int fast, double *d_u,
                            double *d_w, int *d_hits, cudaStream_t st) {
@@ -427,6 +471,13 @@ static void launch_svd_u_g(const double *d_a, long long nmat, int n, int fast, d
 cudaError_t launch_svd_u(const double *d_a, long long nmat, int n, int lanes, int fast,
                          double *d_u, double *d_w, int *d_hits, cudaStream_t st) {
   if (nmat <= 0) return cudaSuccess;
+  if (n == 9) {
+    if (lanes == 1)
+      launch_svd_u9<0>(d_a, nmat, fast, d_u, d_w, d_hits, st);
+    else
+      launch_svd_u9<1>(d_a, nmat, fast, d_u, d_w, d_hits, st);
+    return cudaGetLastError();
+  }
   switch (lanes) {
     case 1: launch_svd_u_g<1>(d_a, nmat, n, fast, d_u, d_w, d_hits, st); break;
     case 2: launch_svd_u_g<2>(d_a, nmat, n, fast, d_u, d_w, d_hits, st); break;
