@@ -123,8 +123,9 @@ struct me_plan {
   int obs_w = 0;
   DevBuf d_slot_obs;
   int grid_jac = 0, grid_trial = 0, grid_svd = 0, grid_fin = 0;
+  int sms = 0;
   // pixels in flight at or below which, with the queue empty, the tail kernel
-  // finishes the batch (-1: half a wave of its warps; 0: rounds only)
+  // finishes the batch (-1: kTailPerSm per SM; 0: rounds only)
   int tail_slots = -1;
   // largest lane group per slot in the rounds once the queue is empty (1: one
   // thread per slot throughout)
@@ -427,6 +428,7 @@ extern "C" int me_plan_create(const me_config *cfg, const double *lambda, int nl
   p->grid_trial = me::round_grid(p->precision, 1, device);
   p->grid_svd = me::round_grid(p->precision, 2, device);
   p->grid_fin = me::round_grid(p->precision, 3, device);
+  cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, device);
   p->grid = p->grid_trial;
   if (cudaMallocHost((void **)&p->h_poll, 2 * sizeof(unsigned long long)) != cudaSuccess ||
       cudaMallocHost((void **)&p->h_feed, kMaxFeedChunks * sizeof(unsigned long long)) !=
@@ -864,13 +866,13 @@ int run_queue(me_plan *p, const me::InvertArgs &A, cudaStream_t st, long long &r
       ggrids[2] = p->P.npar == 9 ? me::svd_grid(9, p->grid_svd, W)
                                  : (int)std::min<long long>(p->grid_trial, need);
     }
-    // default: half a wave of the tail kernel's warps
-    const int tail = p->tail_slots < 0 ? p->grid_fin * (me::kBlock / 32) / 2 : p->tail_slots;
+    const int tail = p->tail_slots < 0 ? p->sms * me::kTailPerSm : p->tail_slots;
     if (drained && busy <= tail) {
-      // the queue is empty and few pixels remain: one warp per pixel to the end
+      // the queue is empty and few pixels remain: each goes to its end on its own
       int *cursor = S.busy + 1;
       CK(cudaMemsetAsync(cursor, 0, sizeof(int), st));
-      const int g = std::min(p->grid_fin, (busy + me::kBlock / 32 - 1) / (me::kBlock / 32));
+      const int per = me::finish_pixels(p->precision);  // pixels per CTA
+      const int g = std::min(p->grid_fin, (busy + per - 1) / per);
       cudaEvent_t *ev = nullptr;
       if (p->profile) {
         // event counts the rounds did, to attribute the rest to the tail
@@ -885,7 +887,7 @@ int run_queue(me_plan *p, const me::InvertArgs &A, cudaStream_t st, long long &r
           CK(cudaEventRecord(ev[0], st));
         }
       }
-      CK(me::launch_finish(p->precision, p->P, A, S, cursor, std::max(g, 1), st));
+      CK(me::launch_finish(p->precision, p->P, A, S, parity, cursor, std::max(g, 1), st));
       if (ev) CK(cudaEventRecord(ev[1], st));
       trace_poll(p, rounds, (long long)p->h_poll[0], busy, 0);
       p->finish_launches++;
@@ -1562,11 +1564,11 @@ extern "C" int me_plan_autotune(me_plan *p, const double *d_prof, long npix, voi
   std::vector<Knob> knobs = {
       {&p->window, {w0 / 2, w0, w0 * 2}},
       {&p->max_group, {1, 4, 8, 16, 32}},
-      // the tail kernel's threshold: none, a quarter, half (the default), one
-      // and two waves of its warps
+      // the tail kernel's threshold: none, half, the default, two and four
+      // times it
       {&p->tail_slots,
-       {0, p->grid_fin * (me::kBlock / 32) / 4, -1, p->grid_fin * (me::kBlock / 32),
-        p->grid_fin * (me::kBlock / 32) * 2}},
+       {0, p->sms * me::kTailPerSm / 2, -1, p->sms * me::kTailPerSm * 2,
+        p->sms * me::kTailPerSm * 4}},
       {&p->svd_lanes, {1, 2}},
       // the Jacobian / trial kernels' variant: 64, 128 or 256 pixels per CTA,
       // the wavelength grid staged in shared memory, no reciprocal table, the

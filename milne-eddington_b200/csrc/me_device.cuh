@@ -1555,6 +1555,440 @@ __device__ __noinline__ int gr_svd_u(double *a, int n, double *w, double *rv1) {
 #undef R_
 }
 
+// a * a + b * b with one of the squares fused into the sum: FORM 0 rounds
+// b * b, FORM 1 rounds a * a.
+template <int FORM>
+__device__ __forceinline__ double sum_sq(double a, double b) {
+  return FORM == 0 ? __fma_rn(a, a, __dmul_rn(b, b)) : __fma_rn(b, b, __dmul_rn(a, a));
+}
+
+// pythag_d with that choice.
+template <int FORM>
+__device__ __forceinline__ double pythag_form(double a, double b) {
+  const double aa = fabs(a), ab = fabs(b);
+  const double mx = aa > ab ? aa : ab;
+  if (mx == 0) return 0;
+  if (mx < 1e150) return sqrt(sum_sq<FORM>(a, b));
+  const double mn = aa > ab ? ab : aa;
+  const double r = mn / mx;
+  return mx * sqrt(__fma_rn(r, r, 1.0));
+}
+// givens_radius in gr_svd9: the radius z and its reciprocal, then c = a / z and
+// s = b / z.  radius_slow is its whole test, out of line.
+template <int FORM, bool FAST>
+static __device__ __noinline__ double2 radius_slow(double a, double b, double q) {
+  if constexpr (FAST) {
+    if (q > 1e-290 && q < 1e290) {
+      const double r = rsqrt(q);
+      return make_double2(__dmul_rn(q, r), r);
+    }
+  }
+  const double z = pythag_form<FORM>(a, b);
+  return make_double2(z, 1.0 / z);
+}
+// The exponent window is tested on q's high word, an integer compare beside
+// the reciprocal square root: 2^-963 <= q < 2^963 lies inside givens_radius's
+// range, and whatever is outside goes through givens_radius's own test.
+// KEEP: c and s keep their values where the radius is zero (the reference's
+// `if (z)`), instead of a / 0 and b / 0.
+template <int FORM, bool FAST, bool KEEP>
+__device__ __forceinline__ double radius9(double a, double b, double &c, double &s) {
+  const double q = sum_sq<FORM>(a, b);
+  if constexpr (FAST) {
+    const double r = rsqrt(q);
+    double z = __dmul_rn(q, r);
+    double c1 = __dmul_rn(a, r), s1 = __dmul_rn(b, r);
+    const unsigned hi = (unsigned)__double2hiint(q);
+    if (__builtin_expect(hi - 0x03c00000u >= 0x7c200000u - 0x03c00000u, 0)) {
+      const double2 e = radius_slow<FORM, true>(a, b, q);
+      z = e.x;
+      c1 = KEEP && z == 0.0 ? c : __dmul_rn(a, e.y);
+      s1 = KEEP && z == 0.0 ? s : __dmul_rn(b, e.y);
+    }
+    c = c1;
+    s = s1;
+    return z;
+  }
+  const double z = pythag_form<FORM>(a, b);
+  const double inv = 1.0 / z;
+  if (!KEEP || z != 0.0) {
+    c = __dmul_rn(a, inv);
+    s = __dmul_rn(b, inv);
+  }
+  return z;
+}
+
+// nonzero: q lies outside radius9's exponent window
+__device__ __forceinline__ unsigned outside9(double q) {
+  return (unsigned)__double2hiint(q) - 0x03c00000u >= 0x7c200000u - 0x03c00000u;
+}
+
+// The cancellation of gr_svd9's QR phase (w[l - 1] negligible: rank-deficient
+// matrices), rare, on a copy in local memory with run-time indices.
+template <bool FAST, int STR>
+static __device__ __noinline__ void svd9_cancel(double *t, int rows, double *w, double *rv1,
+                                                int l, int k, double anorm) {
+  const int nm = l - 1;
+  double c = 0.0, s = 1.0;
+  for (int i = l; i <= k; i++) {
+    const double f = __dmul_rn(s, rv1[i * STR]);
+    rv1[i * STR] = __dmul_rn(c, rv1[i * STR]);
+    if (__dadd_rn(fabs(f), anorm) == anorm) break;
+    const double g = w[i * STR];
+    double fi;
+    w[i * STR] = radius9<0, FAST, false>(f, g, fi, c);
+    s = -fi;
+    for (int j = 0; j < rows; j++) {
+      const double y = t[j * 9 + nm], z = t[j * 9 + i];
+      t[j * 9 + nm] = __fma_rn(y, c, __dmul_rn(z, s));
+      t[j * 9 + i] = __fma_rn(z, c, -__dmul_rn(y, s));
+    }
+  }
+}
+
+// gr_svd_u for a 9 x 9 matrix (no parameter fixed, the common case), one
+// thread per matrix: the matrix in registers, w and rv1 in this thread's
+// columns of shared memory (element i at [i * STR]), and 16 more doubles there
+// (cs) for a sweep's rotations.
+//
+// What bounds it is the latency of the sweeps' scalar chain (two dependent
+// reciprocal square roots per rotation) at the eight warps per SM that the
+// registers allow, so everything else is kept out of its way:
+//   * the Householder phase and the accumulation are unrolled: every index of
+//     A is a constant, the updates of a step's columns interleave, and no
+//     operand makes a round trip through shared memory;
+//   * the QR phase is one loop over sweeps.  Block start l and end k are
+//     run-time values of each thread, so a warp's matrices go through their
+//     own sweeps without meeting at each block end; the splits come from two
+//     bit masks of negligible entries instead of a scan;
+//   * the chain of a sweep is a short rolled loop (it stays in the nearest
+//     instruction cache) that records its rotations; they are applied to A
+//     afterwards by code unrolled over the column and predicated on
+//     l <= column < k.  Unrolling the chain too, or a copy of it per k, makes
+//     a code that instruction fetch cannot feed.
+// Measured on a B200, FAST: one 9 x 9 normal matrix 37 us (one thread in
+// shared memory 95, 32 lanes 59), 131072 of them 193 us = 680 M/s (506 us, 259
+// M/s, one thread in shared memory; 608 us with four lanes), as many
+// orthogonal ones 249 us (781).  8.8 k cycles are the Householder phase, 3.1 k
+// the accumulation, about 300 a rotation and 620 a shift.
+//
+// Every multiply-add is written out, since the results feed an LM that
+// amplifies the last bit: FORM 0 gives gr_svd_u's bits, FORM 1
+// gr_svd_u_grp's, which the compiler fuses differently in the chase's first
+// radius alone.  A NaN matrix, for which no negligible entry is found, is
+// left unrotated.
+constexpr int kSvd9Words = 9 + 9 + 16;  // doubles of shared memory per thread: w, rv1, cs
+
+// The Householder reduction and the accumulation of the left-hand
+// transformations into A; returns anorm.
+template <int STR>
+__device__ __forceinline__ double svd9_reduce(double (&A)[9][9], double *w, double *rv1) {
+  constexpr int n = 9, m = 9;
+  double anorm = 0., g = 0., scale = 0.;
+#pragma unroll
+  for (int i = 0; i < n; i++) {
+    const int l = i + 1;
+    const double rvi = __dmul_rn(scale, g);
+    rv1[i * STR] = rvi;
+    double s = 0.0;
+    g = scale = 0.0;
+#pragma unroll
+    for (int k = i; k < m; k++) scale = __dadd_rn(scale, fabs(A[k][i]));
+    if (scale != 0.0) {
+      const double is = 1.0 / scale;
+#pragma unroll
+      for (int k = i; k < m; k++) {
+        A[k][i] = __dmul_rn(A[k][i], is);
+        s = __fma_rn(A[k][i], A[k][i], s);
+      }
+      const double f = A[i][i];
+      g = f >= 0 ? -sqrt(s) : sqrt(s);
+      const double h = __fma_rn(f, g, -s);
+      A[i][i] = __dsub_rn(f, g);
+      const double ih = 1.0 / h;
+#pragma unroll
+      for (int j = l; j < n; j++) {
+        double sj = 0.0;
+#pragma unroll
+        for (int k = i; k < m; k++) sj = __fma_rn(A[k][i], A[k][j], sj);
+        const double fj = __dmul_rn(sj, ih);
+#pragma unroll
+        for (int k = i; k < m; k++) A[k][j] = __fma_rn(fj, A[k][i], A[k][j]);
+      }
+#pragma unroll
+      for (int k = i; k < m; k++) A[k][i] = __dmul_rn(A[k][i], scale);
+    }
+    const double wi = __dmul_rn(scale, g);
+    w[i * STR] = wi;
+    s = 0.0;
+    g = scale = 0.0;
+    if (i != n - 1) {
+#pragma unroll
+      for (int k = l; k < n; k++) scale = __dadd_rn(scale, fabs(A[i][k]));
+      if (scale != 0.0) {
+        const double is = 1.0 / scale;
+#pragma unroll
+        for (int k = l; k < n; k++) {
+          A[i][k] = __dmul_rn(A[i][k], is);
+          s = __fma_rn(A[i][k], A[i][k], s);
+        }
+        const double f = A[i][l];
+        g = f >= 0 ? -sqrt(s) : sqrt(s);
+        const double h = __fma_rn(f, g, -s);
+        A[i][l] = __dsub_rn(f, g);
+        const double ih = 1.0 / h;
+        double r[9];
+#pragma unroll
+        for (int k = l; k < n; k++) r[k] = __dmul_rn(A[i][k], ih);
+#pragma unroll
+        for (int j = l; j < m; j++) {
+          double sj = 0.0;
+#pragma unroll
+          for (int k = l; k < n; k++) sj = __fma_rn(A[j][k], A[i][k], sj);
+#pragma unroll
+          for (int k = l; k < n; k++) A[j][k] = __fma_rn(sj, r[k], A[j][k]);
+        }
+#pragma unroll
+        for (int k = l; k < n; k++) A[i][k] = __dmul_rn(A[i][k], scale);
+      }
+    }
+    const double t = __dadd_rn(fabs(wi), fabs(rvi));
+    if (anorm < t) anorm = t;
+  }
+  // accumulation of the left-hand transformations into U
+#pragma unroll
+  for (int i = n - 1; i >= 0; i--) {
+    const int l = i + 1;
+    double gi = w[i * STR];
+#pragma unroll
+    for (int j = l; j < n; j++) A[i][j] = 0.0;
+    if (gi != 0.0) {
+      gi = 1.0 / gi;
+      const double iaii = 1.0 / A[i][i];
+#pragma unroll
+      for (int j = l; j < n; j++) {
+        double sj = 0.0;
+#pragma unroll
+        for (int k = l; k < m; k++) sj = __fma_rn(A[k][i], A[k][j], sj);
+        const double fj = __dmul_rn(__dmul_rn(sj, iaii), gi);
+#pragma unroll
+        for (int k = i; k < m; k++) A[k][j] = __fma_rn(fj, A[k][i], A[k][j]);
+      }
+#pragma unroll
+      for (int j = i; j < m; j++) A[j][i] = __dmul_rn(A[j][i], gi);
+    } else {
+#pragma unroll
+      for (int j = i; j < m; j++) A[j][i] = 0.0;
+    }
+    A[i][i] = __dadd_rn(A[i][i], 1.0);
+  }
+  return anorm;
+}
+
+// The implicit-shift QR sweeps, applied to R rows of U in Q.  stop() is asked
+// before each sweep; the sweeps are left when it says so.  Returns 1 when a
+// singular value needed more than 50 sweeps.
+template <int FORM, bool FAST, int STR, int R, class Stop>
+__device__ __forceinline__ int svd9_sweeps(double (&Q)[R][9], double *w, double *rv1, double *cs,
+                                           double anorm, Stop stop) {
+  constexpr int n = 9;
+  int hit = 0;
+  int k = n - 1, its = 0;
+  while (k >= 0) {
+    if (stop()) break;
+    // bit i of zr: rv1[i] is negligible; bit i + 1 of zw: w[i] is
+    unsigned zr = 0, zw = 0;
+#pragma unroll
+    for (int i = 0; i < n; i++) {
+      if (__dadd_rn(fabs(rv1[i * STR]), anorm) == anorm) zr |= 1u << i;
+      if (__dadd_rn(fabs(w[i * STR]), anorm) == anorm) zw |= 2u << i;
+    }
+    int l;
+    bool cancel = false;
+    while (true) {
+      const unsigned z = (zr | zw) & ((2u << k) - 1u);
+      l = z ? 31 - __clz(z) : 0;
+      cancel = z && !((zr >> l) & 1u);
+      if (cancel || l != k) break;
+      if (w[k * STR] < 0.0) w[k * STR] = -w[k * STR];
+      its = 0;
+      if (--k < 0) break;
+    }
+    if (k < 0) break;
+    if (cancel) {
+      double t[R * 9];
+#pragma unroll
+      for (int r = 0; r < R; r++)
+#pragma unroll
+        for (int c = 0; c < n; c++) t[r * 9 + c] = Q[r][c];
+      svd9_cancel<FAST, STR>(t, R, w, rv1, l, k, anorm);
+#pragma unroll
+      for (int r = 0; r < R; r++)
+#pragma unroll
+        for (int c = 0; c < n; c++) Q[r][c] = t[r * 9 + c];
+      if (l == k) {
+        if (w[k * STR] < 0.0) w[k * STR] = -w[k * STR];
+        its = 0;
+        k--;
+        continue;
+      }
+    }
+    if (its == 49) hit = 1;
+    double f, x, c = 1.0, s = 1.0;
+    {
+      x = w[l * STR];
+      const double z = w[k * STR], y = w[(k - 1) * STR];
+      const double gq = rv1[(k - 1) * STR], h = rv1[k * STR];
+      f = __fma_rn(__dsub_rn(y, z), __dadd_rn(y, z),
+                   __dmul_rn(__dsub_rn(gq, h), __dadd_rn(gq, h))) /
+          __dmul_rn(__dmul_rn(2.0, h), y);
+      const double p = pythag_form<0>(f, 1.0);
+      f = __fma_rn(__dsub_rn(x, z), __dadd_rn(x, z),
+                   __dmul_rn(h, __dsub_rn(y / __dadd_rn(f, f >= 0.0 ? p : -p), h))) /
+          x;
+    }
+    // the scalar chain of the sweep; the next step's rv1 and w entries are
+    // loaded a step ahead.  With FAST a step takes no branch: one whose radii
+    // leave the exponent window is done again by slow_step.
+    double gn = rv1[(l + 1) * STR], yn = w[(l + 1) * STR];
+    int j = l;
+    while (true) {
+      unsigned out = 0;
+      double f0, x0, c0, s0, g0, y0;
+#pragma unroll 1
+      do {
+        double g1 = gn, y = yn, z;
+        const int i = (j + 2 < n ? j + 2 : n - 1) * STR;
+        gn = rv1[i];
+        yn = w[i];
+        f0 = f, x0 = x, c0 = c, s0 = s, g0 = g1, y0 = y;
+        double h = __dmul_rn(s, g1);
+        g1 = __dmul_rn(g1, c);
+        if constexpr (FAST) {
+          const double q = sum_sq<FORM>(f, h), r = rsqrt(q);
+          out = outside9(q);
+          z = __dmul_rn(q, r);
+          c = __dmul_rn(f, r);
+          s = __dmul_rn(h, r);
+        } else {
+          z = pythag_form<FORM>(f, h);
+          c = f / z;
+          s = h / z;
+        }
+        rv1[j * STR] = z;
+        f = __fma_rn(x, c, __dmul_rn(g1, s));
+        g1 = __fma_rn(g1, c, -__dmul_rn(x, s));
+        h = __dmul_rn(y, s);
+        y = __dmul_rn(y, c);
+        if constexpr (FAST) {
+          const double q = sum_sq<1>(f, h), r = rsqrt(q);
+          out |= outside9(q);
+          z = __dmul_rn(q, r);
+          c = __dmul_rn(f, r);
+          s = __dmul_rn(h, r);
+        } else {
+          z = radius9<1, false, true>(f, h, c, s);
+        }
+        w[j * STR] = z;
+        cs[j * 2 * STR] = c;
+        cs[(j * 2 + 1) * STR] = s;
+        f = FAST ? __fma_rn(c, g1, __dmul_rn(s, y)) : __fma_rn(s, y, __dmul_rn(c, g1));
+        x = __fma_rn(c, y, -__dmul_rn(s, g1));
+        j++;
+      } while (j < k && !out);
+      if (!out) break;
+      j--;
+      f = f0, x = x0, c = c0, s = s0;
+      {
+        double h = __dmul_rn(s, g0), g1 = __dmul_rn(g0, c), y = y0;
+        double z = radius9<FORM, FAST, false>(f, h, c, s);
+        rv1[j * STR] = z;
+        f = __fma_rn(x, c, __dmul_rn(g1, s));
+        g1 = __fma_rn(g1, c, -__dmul_rn(x, s));
+        h = __dmul_rn(y, s);
+        y = __dmul_rn(y, c);
+        z = radius9<1, FAST, true>(f, h, c, s);
+        w[j * STR] = z;
+        cs[j * 2 * STR] = c;
+        cs[(j * 2 + 1) * STR] = s;
+        f = __fma_rn(c, g1, __dmul_rn(s, y));
+        x = __fma_rn(c, y, -__dmul_rn(s, g1));
+      }
+      if (++j >= k) break;
+    }
+    rv1[l * STR] = 0.0;
+    rv1[k * STR] = f;
+    w[k * STR] = x;
+    // its rotations, on columns j and j + 1 of A
+    double nc = cs[0], ns = cs[STR];
+#pragma unroll
+    for (int q = 0; q < n - 1; q++) {
+      const double rc = nc, rs = ns;
+      if (q < n - 2) {
+        nc = cs[(q + 1) * 2 * STR];
+        ns = cs[(q * 2 + 3) * STR];
+      }
+      if (q >= l && q < k) {
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+          const double y = Q[r][q], z = Q[r][q + 1];
+          Q[r][q] = __fma_rn(y, rc, __dmul_rn(z, rs));
+          Q[r][q + 1] = __fma_rn(z, rc, -__dmul_rn(y, rs));
+        }
+      }
+    }
+    if (++its == 50) {
+      its = 0;
+      k--;
+    }
+  }
+  return hit;
+}
+
+struct NeverStop {
+  __device__ __forceinline__ bool operator()() const { return false; }
+};
+
+template <int FORM, bool FAST, int STR>
+__device__ __forceinline__ int gr_svd9(double (&A)[9][9], double *w, double *rv1, double *cs) {
+  const double anorm = svd9_reduce<STR>(A, w, rv1);
+  return svd9_sweeps<FORM, FAST, STR, 9>(A, w, rv1, cs, anorm, NeverStop());
+}
+
+// gr_svd9 of one matrix by a warp, for the least latency: every lane reduces
+// the matrix (from shared memory, row-major) and runs the sweeps' chain, lane r
+// < 9 turns row r of U.  w, rv1, cs: this lane's own (stride STR).  The rows
+// go to u.
+template <int FORM, bool FAST, int STR, class Stop>
+__device__ __forceinline__ int gr_svd9_warp(const double *a, double *u, double *w, double *rv1,
+                                            double *cs, int lane, Stop stop) {
+  double q[1][9];
+  double anorm;
+  {
+    double A[9][9];
+#pragma unroll
+    for (int r = 0; r < 9; r++)
+#pragma unroll
+      for (int c = 0; c < 9; c++) A[r][c] = a[r * 9 + c];
+    anorm = svd9_reduce<STR>(A, w, rv1);
+#pragma unroll
+    for (int c = 0; c < 9; c++) {
+      q[0][c] = A[0][c];
+#pragma unroll
+      for (int r = 1; r < 9; r++)
+        if (lane == r) q[0][c] = A[r][c];
+    }
+  }
+  const int hit = svd9_sweeps<FORM, FAST, STR, 1>(q, w, rv1, cs, anorm, stop);
+  __syncwarp();  // every lane has read a
+  if (lane < 9) {
+#pragma unroll
+    for (int c = 0; c < 9; c++) u[lane * 9 + c] = q[0][c];
+  }
+  __syncwarp();
+  return hit;
+}
+
 // gr_svd_u for a group of G consecutive lanes of a warp (G a power of two,
 // `mask` the group's lanes), the matrix row-major in the group's shared
 // memory (stride 1): the vector loops of each update are spread over the
@@ -1565,6 +1999,12 @@ __device__ __noinline__ int gr_svd_u(double *a, int n, double *w, double *rv1) {
 // changes.  w [n] is private to the lane.  All lanes of the group call it.
 template <int G, bool FAST = false>
 __device__ __noinline__ int gr_svd_u_grp(double *a, int n, double *w, int lane, unsigned mask) {
+  if constexpr (G == 32) {
+    if (n == 9) {  // the same bits in less time
+      double rv1[9], cs[16];
+      return gr_svd9_warp<1, FAST, 1>(a, a, w, rv1, cs, lane, NeverStop());
+    }
+  }
 #define A_(i, j) a[(i) * n + (j)]
 #define GSYNC()                  \
   do {                           \
@@ -1791,384 +2231,6 @@ __device__ __noinline__ int gr_svd_u_grp(double *a, int n, double *w, int lane, 
 #undef FOR9
 #undef GSYNC
 #undef A_
-}
-
-// a * a + b * b with one of the squares fused into the sum: FORM 0 rounds
-// b * b, FORM 1 rounds a * a.
-template <int FORM>
-__device__ __forceinline__ double sum_sq(double a, double b) {
-  return FORM == 0 ? __fma_rn(a, a, __dmul_rn(b, b)) : __fma_rn(b, b, __dmul_rn(a, a));
-}
-
-// pythag_d with that choice.
-template <int FORM>
-__device__ __forceinline__ double pythag_form(double a, double b) {
-  const double aa = fabs(a), ab = fabs(b);
-  const double mx = aa > ab ? aa : ab;
-  if (mx == 0) return 0;
-  if (mx < 1e150) return sqrt(sum_sq<FORM>(a, b));
-  const double mn = aa > ab ? ab : aa;
-  const double r = mn / mx;
-  return mx * sqrt(__fma_rn(r, r, 1.0));
-}
-// givens_radius in gr_svd9: the radius z and its reciprocal, then c = a / z and
-// s = b / z.  radius_slow is its whole test, out of line.
-template <int FORM, bool FAST>
-static __device__ __noinline__ double2 radius_slow(double a, double b, double q) {
-  if constexpr (FAST) {
-    if (q > 1e-290 && q < 1e290) {
-      const double r = rsqrt(q);
-      return make_double2(__dmul_rn(q, r), r);
-    }
-  }
-  const double z = pythag_form<FORM>(a, b);
-  return make_double2(z, 1.0 / z);
-}
-// The exponent window is tested on q's high word, an integer compare beside
-// the reciprocal square root: 2^-963 <= q < 2^963 lies inside givens_radius's
-// range, and whatever is outside goes through givens_radius's own test.
-// KEEP: c and s keep their values where the radius is zero (the reference's
-// `if (z)`), instead of a / 0 and b / 0.
-template <int FORM, bool FAST, bool KEEP>
-__device__ __forceinline__ double radius9(double a, double b, double &c, double &s) {
-  const double q = sum_sq<FORM>(a, b);
-  if constexpr (FAST) {
-    const double r = rsqrt(q);
-    double z = __dmul_rn(q, r);
-    double c1 = __dmul_rn(a, r), s1 = __dmul_rn(b, r);
-    const unsigned hi = (unsigned)__double2hiint(q);
-    if (__builtin_expect(hi - 0x03c00000u >= 0x7c200000u - 0x03c00000u, 0)) {
-      const double2 e = radius_slow<FORM, true>(a, b, q);
-      z = e.x;
-      c1 = KEEP && z == 0.0 ? c : __dmul_rn(a, e.y);
-      s1 = KEEP && z == 0.0 ? s : __dmul_rn(b, e.y);
-    }
-    c = c1;
-    s = s1;
-    return z;
-  }
-  const double z = pythag_form<FORM>(a, b);
-  const double inv = 1.0 / z;
-  if (!KEEP || z != 0.0) {
-    c = __dmul_rn(a, inv);
-    s = __dmul_rn(b, inv);
-  }
-  return z;
-}
-
-// nonzero: q lies outside radius9's exponent window
-__device__ __forceinline__ unsigned outside9(double q) {
-  return (unsigned)__double2hiint(q) - 0x03c00000u >= 0x7c200000u - 0x03c00000u;
-}
-
-// The cancellation of gr_svd9's QR phase (w[l - 1] negligible: rank-deficient
-// matrices), rare, on a copy in local memory with run-time indices.
-template <bool FAST, int STR>
-static __device__ __noinline__ void svd9_cancel(double *t, double *w, double *rv1, int l, int k,
-                                                double anorm) {
-  const int nm = l - 1;
-  double c = 0.0, s = 1.0;
-  for (int i = l; i <= k; i++) {
-    const double f = __dmul_rn(s, rv1[i * STR]);
-    rv1[i * STR] = __dmul_rn(c, rv1[i * STR]);
-    if (__dadd_rn(fabs(f), anorm) == anorm) break;
-    const double g = w[i * STR];
-    double fi;
-    w[i * STR] = radius9<0, FAST, false>(f, g, fi, c);
-    s = -fi;
-    for (int j = 0; j < 9; j++) {
-      const double y = t[j * 9 + nm], z = t[j * 9 + i];
-      t[j * 9 + nm] = __fma_rn(y, c, __dmul_rn(z, s));
-      t[j * 9 + i] = __fma_rn(z, c, -__dmul_rn(y, s));
-    }
-  }
-}
-
-// gr_svd_u for a 9 x 9 matrix (no parameter fixed, the common case), one
-// thread per matrix: the matrix in registers, w and rv1 in this thread's
-// columns of shared memory (element i at [i * STR]), and 16 more doubles there
-// (cs) for a sweep's rotations.
-//
-// What bounds it is the latency of the sweeps' scalar chain (two dependent
-// reciprocal square roots per rotation) at the eight warps per SM that the
-// registers allow, so everything else is kept out of its way:
-//   * the Householder phase and the accumulation are unrolled: every index of
-//     A is a constant, the updates of a step's columns interleave, and no
-//     operand makes a round trip through shared memory;
-//   * the QR phase is one loop over sweeps.  Block start l and end k are
-//     run-time values of each thread, so a warp's matrices go through their
-//     own sweeps without meeting at each block end; the splits come from two
-//     bit masks of negligible entries instead of a scan;
-//   * the chain of a sweep is a short rolled loop (it stays in the nearest
-//     instruction cache) that records its rotations; they are applied to A
-//     afterwards by code unrolled over the column and predicated on
-//     l <= column < k.  Unrolling the chain too, or a copy of it per k, makes
-//     a code that instruction fetch cannot feed.
-// Measured on a B200, FAST: one 9 x 9 normal matrix 37 us (one thread in
-// shared memory 95, 32 lanes 59), 131072 of them 193 us = 680 M/s (506 us, 259
-// M/s, one thread in shared memory; 608 us with four lanes), as many
-// orthogonal ones 249 us (781).  8.8 k cycles are the Householder phase, 3.1 k
-// the accumulation, about 300 a rotation and 620 a shift.
-//
-// Every multiply-add is written out, since the results feed an LM that
-// amplifies the last bit: FORM 0 gives gr_svd_u's bits, FORM 1
-// gr_svd_u_grp's, which the compiler fuses differently in the chase's first
-// radius alone.  A NaN matrix, for which no negligible entry is found, is
-// left unrotated.
-constexpr int kSvd9Words = 9 + 9 + 16;  // doubles of shared memory per thread: w, rv1, cs
-
-template <int FORM, bool FAST, int STR>
-__device__ __forceinline__ int gr_svd9(double (&A)[9][9], double *w, double *rv1, double *cs) {
-  constexpr int n = 9, m = 9;
-  double anorm = 0., g = 0., scale = 0.;
-  int hit = 0;
-#pragma unroll
-  for (int i = 0; i < n; i++) {
-    const int l = i + 1;
-    const double rvi = __dmul_rn(scale, g);
-    rv1[i * STR] = rvi;
-    double s = 0.0;
-    g = scale = 0.0;
-#pragma unroll
-    for (int k = i; k < m; k++) scale = __dadd_rn(scale, fabs(A[k][i]));
-    if (scale != 0.0) {
-      const double is = 1.0 / scale;
-#pragma unroll
-      for (int k = i; k < m; k++) {
-        A[k][i] = __dmul_rn(A[k][i], is);
-        s = __fma_rn(A[k][i], A[k][i], s);
-      }
-      const double f = A[i][i];
-      g = f >= 0 ? -sqrt(s) : sqrt(s);
-      const double h = __fma_rn(f, g, -s);
-      A[i][i] = __dsub_rn(f, g);
-      const double ih = 1.0 / h;
-#pragma unroll
-      for (int j = l; j < n; j++) {
-        double sj = 0.0;
-#pragma unroll
-        for (int k = i; k < m; k++) sj = __fma_rn(A[k][i], A[k][j], sj);
-        const double fj = __dmul_rn(sj, ih);
-#pragma unroll
-        for (int k = i; k < m; k++) A[k][j] = __fma_rn(fj, A[k][i], A[k][j]);
-      }
-#pragma unroll
-      for (int k = i; k < m; k++) A[k][i] = __dmul_rn(A[k][i], scale);
-    }
-    const double wi = __dmul_rn(scale, g);
-    w[i * STR] = wi;
-    s = 0.0;
-    g = scale = 0.0;
-    if (i != n - 1) {
-#pragma unroll
-      for (int k = l; k < n; k++) scale = __dadd_rn(scale, fabs(A[i][k]));
-      if (scale != 0.0) {
-        const double is = 1.0 / scale;
-#pragma unroll
-        for (int k = l; k < n; k++) {
-          A[i][k] = __dmul_rn(A[i][k], is);
-          s = __fma_rn(A[i][k], A[i][k], s);
-        }
-        const double f = A[i][l];
-        g = f >= 0 ? -sqrt(s) : sqrt(s);
-        const double h = __fma_rn(f, g, -s);
-        A[i][l] = __dsub_rn(f, g);
-        const double ih = 1.0 / h;
-        double r[9];
-#pragma unroll
-        for (int k = l; k < n; k++) r[k] = __dmul_rn(A[i][k], ih);
-#pragma unroll
-        for (int j = l; j < m; j++) {
-          double sj = 0.0;
-#pragma unroll
-          for (int k = l; k < n; k++) sj = __fma_rn(A[j][k], A[i][k], sj);
-#pragma unroll
-          for (int k = l; k < n; k++) A[j][k] = __fma_rn(sj, r[k], A[j][k]);
-        }
-#pragma unroll
-        for (int k = l; k < n; k++) A[i][k] = __dmul_rn(A[i][k], scale);
-      }
-    }
-    const double t = __dadd_rn(fabs(wi), fabs(rvi));
-    if (anorm < t) anorm = t;
-  }
-  // accumulation of the left-hand transformations into U
-#pragma unroll
-  for (int i = n - 1; i >= 0; i--) {
-    const int l = i + 1;
-    double gi = w[i * STR];
-#pragma unroll
-    for (int j = l; j < n; j++) A[i][j] = 0.0;
-    if (gi != 0.0) {
-      gi = 1.0 / gi;
-      const double iaii = 1.0 / A[i][i];
-#pragma unroll
-      for (int j = l; j < n; j++) {
-        double sj = 0.0;
-#pragma unroll
-        for (int k = l; k < m; k++) sj = __fma_rn(A[k][i], A[k][j], sj);
-        const double fj = __dmul_rn(__dmul_rn(sj, iaii), gi);
-#pragma unroll
-        for (int k = i; k < m; k++) A[k][j] = __fma_rn(fj, A[k][i], A[k][j]);
-      }
-#pragma unroll
-      for (int j = i; j < m; j++) A[j][i] = __dmul_rn(A[j][i], gi);
-    } else {
-#pragma unroll
-      for (int j = i; j < m; j++) A[j][i] = 0.0;
-    }
-    A[i][i] = __dadd_rn(A[i][i], 1.0);
-  }
-  // implicit-shift QR sweeps
-  int k = n - 1, its = 0;
-  while (k >= 0) {
-    // bit i of zr: rv1[i] is negligible; bit i + 1 of zw: w[i] is
-    unsigned zr = 0, zw = 0;
-#pragma unroll
-    for (int i = 0; i < n; i++) {
-      if (__dadd_rn(fabs(rv1[i * STR]), anorm) == anorm) zr |= 1u << i;
-      if (__dadd_rn(fabs(w[i * STR]), anorm) == anorm) zw |= 2u << i;
-    }
-    int l;
-    bool cancel = false;
-    while (true) {
-      const unsigned z = (zr | zw) & ((2u << k) - 1u);
-      l = z ? 31 - __clz(z) : 0;
-      cancel = z && !((zr >> l) & 1u);
-      if (cancel || l != k) break;
-      if (w[k * STR] < 0.0) w[k * STR] = -w[k * STR];
-      its = 0;
-      if (--k < 0) break;
-    }
-    if (k < 0) break;
-    if (cancel) {
-      double t[81];
-#pragma unroll
-      for (int r = 0; r < m; r++)
-#pragma unroll
-        for (int c = 0; c < n; c++) t[r * 9 + c] = A[r][c];
-      svd9_cancel<FAST, STR>(t, w, rv1, l, k, anorm);
-#pragma unroll
-      for (int r = 0; r < m; r++)
-#pragma unroll
-        for (int c = 0; c < n; c++) A[r][c] = t[r * 9 + c];
-      if (l == k) {
-        if (w[k * STR] < 0.0) w[k * STR] = -w[k * STR];
-        its = 0;
-        k--;
-        continue;
-      }
-    }
-    if (its == 49) hit = 1;
-    double f, x, c = 1.0, s = 1.0;
-    {
-      x = w[l * STR];
-      const double z = w[k * STR], y = w[(k - 1) * STR];
-      const double gq = rv1[(k - 1) * STR], h = rv1[k * STR];
-      f = __fma_rn(__dsub_rn(y, z), __dadd_rn(y, z),
-                   __dmul_rn(__dsub_rn(gq, h), __dadd_rn(gq, h))) /
-          __dmul_rn(__dmul_rn(2.0, h), y);
-      const double p = pythag_form<0>(f, 1.0);
-      f = __fma_rn(__dsub_rn(x, z), __dadd_rn(x, z),
-                   __dmul_rn(h, __dsub_rn(y / __dadd_rn(f, f >= 0.0 ? p : -p), h))) /
-          x;
-    }
-    // the scalar chain of the sweep; the next step's rv1 and w entries are
-    // loaded a step ahead.  With FAST a step takes no branch: one whose radii
-    // leave the exponent window is done again by slow_step.
-    double gn = rv1[(l + 1) * STR], yn = w[(l + 1) * STR];
-    int j = l;
-    while (true) {
-      unsigned out = 0;
-      double f0, x0, c0, s0, g0, y0;
-#pragma unroll 1
-      do {
-        double g1 = gn, y = yn, z;
-        const int i = (j + 2 < n ? j + 2 : n - 1) * STR;
-        gn = rv1[i];
-        yn = w[i];
-        f0 = f, x0 = x, c0 = c, s0 = s, g0 = g1, y0 = y;
-        double h = __dmul_rn(s, g1);
-        g1 = __dmul_rn(g1, c);
-        if constexpr (FAST) {
-          const double q = sum_sq<FORM>(f, h), r = rsqrt(q);
-          out = outside9(q);
-          z = __dmul_rn(q, r);
-          c = __dmul_rn(f, r);
-          s = __dmul_rn(h, r);
-        } else {
-          z = pythag_form<FORM>(f, h);
-          c = f / z;
-          s = h / z;
-        }
-        rv1[j * STR] = z;
-        f = __fma_rn(x, c, __dmul_rn(g1, s));
-        g1 = __fma_rn(g1, c, -__dmul_rn(x, s));
-        h = __dmul_rn(y, s);
-        y = __dmul_rn(y, c);
-        if constexpr (FAST) {
-          const double q = sum_sq<1>(f, h), r = rsqrt(q);
-          out |= outside9(q);
-          z = __dmul_rn(q, r);
-          c = __dmul_rn(f, r);
-          s = __dmul_rn(h, r);
-        } else {
-          z = radius9<1, false, true>(f, h, c, s);
-        }
-        w[j * STR] = z;
-        cs[j * 2 * STR] = c;
-        cs[(j * 2 + 1) * STR] = s;
-        f = FAST ? __fma_rn(c, g1, __dmul_rn(s, y)) : __fma_rn(s, y, __dmul_rn(c, g1));
-        x = __fma_rn(c, y, -__dmul_rn(s, g1));
-        j++;
-      } while (j < k && !out);
-      if (!out) break;
-      j--;
-      f = f0, x = x0, c = c0, s = s0;
-      {
-        double h = __dmul_rn(s, g0), g1 = __dmul_rn(g0, c), y = y0;
-        double z = radius9<FORM, FAST, false>(f, h, c, s);
-        rv1[j * STR] = z;
-        f = __fma_rn(x, c, __dmul_rn(g1, s));
-        g1 = __fma_rn(g1, c, -__dmul_rn(x, s));
-        h = __dmul_rn(y, s);
-        y = __dmul_rn(y, c);
-        z = radius9<1, FAST, true>(f, h, c, s);
-        w[j * STR] = z;
-        cs[j * 2 * STR] = c;
-        cs[(j * 2 + 1) * STR] = s;
-        f = __fma_rn(c, g1, __dmul_rn(s, y));
-        x = __fma_rn(c, y, -__dmul_rn(s, g1));
-      }
-      if (++j >= k) break;
-    }
-    rv1[l * STR] = 0.0;
-    rv1[k * STR] = f;
-    w[k * STR] = x;
-    // its rotations, on columns j and j + 1 of A
-    double nc = cs[0], ns = cs[STR];
-#pragma unroll
-    for (int q = 0; q < n - 1; q++) {
-      const double rc = nc, rs = ns;
-      if (q < n - 2) {
-        nc = cs[(q + 1) * 2 * STR];
-        ns = cs[(q * 2 + 3) * STR];
-      }
-      if (q >= l && q < k) {
-#pragma unroll
-        for (int r = 0; r < m; r++) {
-          const double y = A[r][q], z = A[r][q + 1];
-          A[r][q] = __fma_rn(y, rc, __dmul_rn(z, rs));
-          A[r][q + 1] = __fma_rn(z, rc, -__dmul_rn(y, rs));
-        }
-      }
-    }
-    if (++its == 50) {
-      its = 0;
-      k--;
-    }
-  }
-  return hit;
 }
 
 // x = V diag(1/w) U^T b, skipping w <= 1e-50 (svbksb, SVD_TEMPLATE.h:348-406).

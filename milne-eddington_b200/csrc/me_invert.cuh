@@ -1122,6 +1122,644 @@ __global__ void __launch_bounds__(kBlock, 1) finish_kernel(const __grid_constant
 }
 
 // ---------------------------------------------------------------------------
+// The tail of FP32 plans: with few pixels left, a batch's time is
+// the longest remaining chain of LM steps, and a step's time is its latency.
+// tail_kernel takes the remaining slots, one CTA per pixel (an atomic cursor
+// over the next round's lists), and runs each to completion.  A CTA is
+// TailShape::kSynth warps that synthesise, one point per lane, and one warp
+// that decomposes:
+//   * the per-point terms are staged in shared memory and every sum over the
+//     wavelengths is formed by one lane in the thread-serial order.  With an
+//     instrument filter the points are the sub-wavelengths, and each observed
+//     value is summed from them in order, so all lanes have work on a grid of
+//     a few wavelengths;
+//   * the factors that a run of rejected trials needs (H's U, then the U of
+//     that U, ...) do not depend on the trials' outcome: from the first
+//     rejection on the decomposing warp makes the next trial's factor while
+//     the current trial is synthesised, and drops it when that is accepted.
+//     (Running ahead of the first trial too costs more, in dropping the
+//     factor at each accepted step, than it saves);
+//   * the slot's state sits in shared memory (a Slots view with W = 1), so the
+//     scalar transitions make no round trips to the L2 cache.
+// The arithmetic is the one-warp-per-pixel form's (deriv_warp, forward_warp,
+// solve_slot with lanes) operation for operation.  Waits between the warps are
+// bounded; one that runs out ends the pixel with flag 8, which the host
+// reports as ME_ERR_TIMEOUT.
+// FP64 plans run finish_kernel above: inlined here, the FP64 synthesis is fused
+// differently by the compiler, and the LM amplifies the last bit.
+// Measured (FP32, Fe I 15648, 60 wavelengths, an LM step of the longest chain):
+// 23 us with 20 pixels in flight and 25 with 590, against 42 and 43 with one
+// warp per pixel; the filtered Fe I 6173 grid 24 against 48.  Of an accepted
+// step's 95 k cycles about 53 k are the decomposition, 17 k the synthesis with
+// Jacobian and its sums, 8 k the trial's synthesis.
+// ---------------------------------------------------------------------------
+template <class T, bool FILT>
+struct TailShape {
+  // a plain grid: one synthesising warp, since four CTAs of 64 per SM then
+  // hold every pixel the tail is left with at once; a filtered one has a few
+  // dozen points per wavelength and gets three
+  static constexpr int kSynth = FILT ? 3 : 1;
+  static constexpr int kPoints = 32 * kSynth;
+  static constexpr int kThreads = kPoints + 32;
+};
+
+// What the two sides of a tail CTA tell each other (shared memory).
+struct TailCtl {
+  int gen;   // chain of factors asked for (raised with each new start matrix)
+  int base;  // the start matrix is the factor U_base (0: H)
+  int want;  // the last factor asked for
+  int quit;
+  int pub_gen, pub_k;  // factors of chain pub_gen up to pub_k are there
+  int item, error;
+};
+
+// One slot's state in shared memory.
+struct TailSlot {
+  long long pix;
+  int state, run, it, tk;
+  unsigned int cnt[4];
+  unsigned char had_trial;
+  double sc[SC_COUNT], guess[9], par[9], pbest[9], jvec[9], ptmp[9];
+};
+
+template <class T, bool FILT>
+struct TailSmem {
+  using Sh = TailShape<T, FILT>;
+  double svd[kSvd9Words * 32];  // the decomposing warp's w, rv1, cs columns
+  double start[81];             // the chain's start matrix
+  double fac[3][81];            // factor k in fac[k % 3]
+  double w[9];                  // singular values of H
+  double R[Sh::kPoints * 4];    // weighted residuals of a batch of points
+  double hg[56];                // the sums: H (45), g (9), chi^2
+  TailSlot slot;
+  TailCtl ctl;
+  int hit[3];
+  T tab[100];
+  T J[Sh::kPoints * 40];        // per point and Stokes parameter: Jacobian row, residual
+  T pt[FILT ? Sh::kPoints * 40 : 1];  // filter: profiles and rows of the sub-wavelengths
+  T part[FILT ? 40 : 1];        // and a wavelength's sums so far, from one batch to the next
+  T rden[Sh::kSynth][kRden];
+};
+
+namespace detail {
+
+constexpr int kTailSpin = 1 << 22;  // polls before a wait gives up (some 0.1 s)
+
+// barrier of the synthesising warps (the decomposing warp runs on its own)
+template <int NS>
+__device__ __forceinline__ void tail_sync() {
+  if (NS == 1)
+    __syncwarp();
+  else
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * NS) : "memory");
+}
+
+// Profiles and Jacobian rows of a filtered grid's wavelengths: points p =
+// (wavelength, sub-wavelength) in order, kPoints at a time; each lane computes
+// one, then each of the 4 (with DERIV 40) entries of the wavelengths they
+// belong to is summed over its sub-wavelengths in order, from zero, by one
+// lane.  emit(iw, e, v): entry e of wavelength iw is complete (e < 4 the
+// profiles, then J[s][k] at 4 + 9 s + k).
+template <class T, bool DERIV, class Emit>
+__device__ __forceinline__ void tail_filter_points(const SynthCall<T> &c, const DevPlan &P,
+                                                   VoigtK<T> &K, const T sw[4], int tid, T *pt,
+                                                   T *part, int first, int last, Emit emit) {
+  using Sh = TailShape<T, true>;
+  constexpr int E = DERIV ? 40 : 4;
+  const int ns = P.nsub;
+  for (int p0 = first * ns; p0 < last * ns; p0 += Sh::kPoints) {
+    const int p = p0 + tid;
+    if (p < last * ns) {
+      T ys[4], Jq[4][9];
+      me_point<T, DERIV>(c, shift_wf<T>(c, P, p), K, sw, ys, DERIV ? Jq : nullptr);
+#pragma unroll
+      for (int s = 0; s < 4; s++) pt[tid * E + s] = ys[s];
+      if (DERIV) {
+#pragma unroll
+        for (int s = 0; s < 4; s++)
+#pragma unroll
+          for (int k = 0; k < 9; k++) pt[tid * E + 4 + s * 9 + k] = Jq[s][k];
+      }
+    }
+    tail_sync<Sh::kSynth>();
+    const int p1 = p0 + Sh::kPoints < last * ns ? p0 + Sh::kPoints : last * ns;
+    const int w0 = p0 / ns, w1 = (p1 - 1) / ns;
+    // a wavelength's sums may come from, and go to, the neighbouring batches:
+    // only its first and only its last one in this batch
+    T carry = T(0);
+    for (int u = tid; u < (w1 - w0 + 1) * E; u += Sh::kPoints) {
+      const int iw = w0 + u / E, e = u % E;
+      const int q0 = iw * ns > p0 ? iw * ns : p0;
+      const int q1 = (iw + 1) * ns < p1 ? (iw + 1) * ns : p1;
+      T v = q0 == iw * ns ? T(0) : part[e];
+      for (int q = q0; q < q1; q++) v += T(P.sub_w[q - iw * ns]) * pt[(q - p0) * E + e];
+      if (q1 == (iw + 1) * ns)
+        emit(iw, e, v);
+      else
+        carry = v;
+    }
+    tail_sync<Sh::kSynth>();
+    if (p1 < (w1 + 1) * ns) {
+      // the batch ends inside wavelength w1: its lanes put the sums by
+      for (int u = tid; u < (w1 - w0 + 1) * E; u += Sh::kPoints)
+        if (u / E == w1 - w0) part[u % E] = carry;
+      tail_sync<Sh::kSynth>();
+    }
+  }
+}
+
+// deriv_pass by the synthesising warps.  H45, g9 and chi^2 / (4 nl) land in
+// sm.hg (all may read after the call).
+template <class T, bool FILT>
+__device__ void deriv_tail(const DevPlan &P, VoigtK<T> &K, T *rden, const double *par,
+                           const double *step, const double *prof, const double sw[4], int tid,
+                           TailSmem<T, FILT> &sm) {
+  using Sh = TailShape<T, FILT>;
+  const int lane = tid & 31;
+  SynthCall<T> c;
+  synth_setup<T>(c, par, P, step);
+  voigt_prepare_warp<T>(K, c.p5, rden, lane);
+  const int nl = P.nl;
+  const T tsw[4] = {T(sw[0]), T(sw[1]), T(sw[2]), T(sw[3])};
+  T *stJ = sm.J;
+  double *stR = sm.R;
+  // this lane's sums (first warp): entries lane and lane + 32 of the 45 of H
+  // (upper triangle, row-major) and the 9 of g, which are minus the products
+  // with column 9, the residual
+  int i0 = 0, j0 = 0, i1 = lane + 32 - 45, j1 = 9;
+  {
+    int idx = 0;
+    for (int i = 0; i < 9; i++)
+      for (int j = i; j < 9; j++, idx++) {
+        if (idx == lane) i0 = i, j0 = j;
+        if (idx == lane + 32) i1 = i, j1 = j;
+      }
+  }
+  if (lane + 32 >= 54) i1 = 0;
+  const bool minus = j1 == 9;
+  T h0 = T(0), h1 = T(0);
+  double chi = 0.0;
+  for (int base = 0; base < nl; base += Sh::kPoints) {
+    const int cnt = nl - base < Sh::kPoints ? nl - base : Sh::kPoints;
+    if constexpr (FILT) {
+      tail_filter_points<T, true>(c, P, K, tsw, tid, sm.pt, sm.part, base, base + cnt,
+                                  [&](int iw, int e, T v) {
+                                    if (e < 4) {
+                                      const double rd =
+                                          ((double)v - __ldg(prof + e * nl + iw)) * sw[e];
+                                      stR[(iw - base) * 4 + e] = rd;
+                                      stJ[(iw - base) * 40 + e * 10 + 9] = T(rd);
+                                    } else {
+                                      const int s = (e - 4) / 9, k = (e - 4) % 9;
+                                      stJ[(iw - base) * 40 + s * 10 + k] = v;
+                                    }
+                                  });
+    } else {
+      const int iw = base + tid;
+      if (iw < nl) {
+        T syn[4], J[4][9];
+        channel_point<T, true, false>(c, P, K, tsw, iw, syn, J);
+#pragma unroll
+        for (int s = 0; s < 4; s++) {
+          const double rd = ((double)syn[s] - __ldg(prof + s * nl + iw)) * sw[s];
+          stR[tid * 4 + s] = rd;
+          stJ[tid * 40 + s * 10 + 9] = T(rd);
+#pragma unroll
+          for (int k = 0; k < 9; k++) stJ[tid * 40 + s * 10 + k] = J[s][k];
+        }
+      }
+    }
+    tail_sync<Sh::kSynth>();
+    if (tid < 32) {
+#pragma unroll 4
+      for (int q = 0; q < cnt; q++) {
+        const double *rq = stR + q * 4;
+        const T *Jq = stJ + q * 40;
+#pragma unroll
+        for (int s = 0; s < 4; s++) {
+          const double rd = rq[s];
+          chi += rd * rd;
+        }
+        h0 += Jq[i0] * Jq[j0] + Jq[10 + i0] * Jq[10 + j0] + Jq[20 + i0] * Jq[20 + j0] +
+              Jq[30 + i0] * Jq[30 + j0];
+        const T t1 = Jq[i1] * Jq[j1] + Jq[10 + i1] * Jq[10 + j1] + Jq[20 + i1] * Jq[20 + j1] +
+                     Jq[30 + i1] * Jq[30 + j1];
+        h1 += minus ? -t1 : t1;
+      }
+    }
+    tail_sync<Sh::kSynth>();
+  }
+  if (tid < 32) {
+    sm.hg[lane] = (double)h0;
+    if (lane + 32 < 54) sm.hg[lane + 32] = (double)h1;
+    if (lane == 0) sm.hg[54] = chi / (4.0 * nl);
+  }
+  tail_sync<Sh::kSynth>();
+}
+
+// forward_pass by the synthesising warps (chi^2 only); every lane of the first
+// gets the result.
+template <class T, bool FILT>
+__device__ double forward_tail(const DevPlan &P, VoigtK<T> &K, T *rden, const double *par,
+                               const double *step, const double *prof, const double sw[4], int tid,
+                               TailSmem<T, FILT> &sm) {
+  using Sh = TailShape<T, FILT>;
+  SynthCall<T> c;
+  synth_setup<T>(c, par, P, step);
+  voigt_prepare_warp<T>(K, c.p5, rden, tid & 31);
+  const T ones[4] = {T(1), T(1), T(1), T(1)};
+  const int nl = P.nl;
+  double *stR = sm.R;
+  double chi = 0.0;
+  for (int base = 0; base < nl; base += Sh::kPoints) {
+    const int cnt = nl - base < Sh::kPoints ? nl - base : Sh::kPoints;
+    if constexpr (FILT) {
+      tail_filter_points<T, false>(c, P, K, ones, tid, sm.pt, sm.part, base, base + cnt,
+                                   [&](int iw, int e, T v) {
+                                     stR[(iw - base) * 4 + e] =
+                                         ((double)v - __ldg(prof + e * nl + iw)) * sw[e];
+                                   });
+    } else {
+      const int iw = base + tid;
+      if (iw < nl) {
+        T syn[4];
+        channel_point<T, false, false>(c, P, K, ones, iw, syn, nullptr);
+#pragma unroll
+        for (int s = 0; s < 4; s++)
+          stR[tid * 4 + s] = ((double)syn[s] - __ldg(prof + s * nl + iw)) * sw[s];
+      }
+    }
+    tail_sync<Sh::kSynth>();
+    if (tid < 32) {
+#pragma unroll 4
+      for (int q = 0; q < cnt; q++)
+#pragma unroll
+        for (int s = 0; s < 4; s++) {
+          const double rd = stR[q * 4 + s];
+          chi += rd * rd;
+        }
+    }
+    tail_sync<Sh::kSynth>();
+  }
+  return chi / (4.0 * nl);
+}
+
+__device__ __forceinline__ int vload(const int *p) { return *(const volatile int *)p; }
+__device__ __forceinline__ void vstore(int *p, int v) { *(volatile int *)p = v; }
+
+// The decomposing warp: the chains of factors the trials ask for.  Factor k of
+// a chain is the U of factor k - 1's decomposition.  The trials ask for factor
+// k while they use factor k - 1 or an earlier one's wait, so three buffers keep
+// what is read, read from and written apart.
+template <class T, bool FILT>
+__device__ void tail_decompose(const DevPlan &P, TailSmem<T, FILT> &sm, int lane) {
+  TailCtl &ctl = sm.ctl;
+  double *w = sm.svd + lane, *rv1 = sm.svd + 9 * 32 + lane, *cs = sm.svd + 18 * 32 + lane;
+  const int n = P.npar;
+  int gen = 0, spins = 0;
+  while (true) {
+    // the next chain (generations only grow, so the wait sees the newest)
+    int g = __shfl_sync(0xffffffffu, vload(&ctl.gen), 0);
+    if (__shfl_sync(0xffffffffu, vload(&ctl.quit), 0)) return;
+    if (g == gen) {
+      if (++spins > kTailSpin) return;  // the trials' side gives up on its own
+      __nanosleep(40);
+      continue;
+    }
+    spins = 0;
+    gen = g;
+    __threadfence_block();
+    const int base = vload(&ctl.base);
+    auto stale = [&]() {
+      return __shfl_sync(0xffffffffu, vload(&ctl.gen) != gen || vload(&ctl.quit), 0) != 0;
+    };
+    for (int k = base + 1;; k++) {
+      int polls = 0;
+      bool drop = false;
+      while (true) {
+        drop = stale();
+        if (drop || __shfl_sync(0xffffffffu, vload(&ctl.want), 0) >= k) break;
+        if (++polls > kTailSpin) return;
+        __nanosleep(40);
+      }
+      if (drop) break;
+      __threadfence_block();
+      const double *a = k == base + 1 ? sm.start : sm.fac[(k - 1) % 3];
+      double *u = sm.fac[k % 3];
+      int hit;
+      if (n == 9) {
+        hit = P.fastg ? gr_svd9_warp<1, true, 32>(a, u, w, rv1, cs, lane, stale)
+                      : gr_svd9_warp<1, false, 32>(a, u, w, rv1, cs, lane, stale);
+        if (k == 1 && lane < 9) {
+          double v = 0.0;
+          for (int i = 0; i < 9; i++)
+            if (i == lane) v = w[i * 32];
+          sm.w[lane] = v;
+        }
+      } else {
+        for (int i = lane; i < n * n; i += 32) u[i] = a[i];
+        __syncwarp();
+        double wl[9];
+        hit = P.fastg ? gr_svd_u_grp<32, true>(u, n, wl, lane, 0xffffffffu)
+                      : gr_svd_u_grp<32, false>(u, n, wl, lane, 0xffffffffu);
+        if (k == 1 && lane == 0)
+          for (int i = 0; i < n; i++) sm.w[i] = wl[i];
+      }
+      __syncwarp();
+      if (lane == 0) {
+        sm.hit[k % 3] = hit;
+        __threadfence_block();
+        // a chain dropped in mid-sweep is published under its own generation,
+        // which nobody waits for
+        vstore(&ctl.pub_k, k);
+        __threadfence_block();
+        vstore(&ctl.pub_gen, gen);
+      }
+      __syncwarp();
+    }
+  }
+}
+
+// solve_slot's trial parameters from the factors of the decomposing warp, by
+// the first synthesising warp.  Returns the decompositions that hit the sweep
+// limit, or -1 when the wait for a factor ran out.
+template <class T, bool FILT>
+__device__ __forceinline__ int tail_solve(const DevPlan &P, const Slots &L,
+                                          TailSmem<T, FILT> &sm, int lane) {
+  const int n = P.npar;
+  const int tk = sm.slot.tk;
+  const int k = tk == 1 ? 1 : tk - 1;
+  const int base = sm.ctl.base, gen = sm.ctl.gen;
+  int hits = 0;
+  const double *a = sm.start;
+  if (k > base) {
+    int polls = 0;
+    while (true) {
+      const bool there = vload(&sm.ctl.pub_gen) == gen && vload(&sm.ctl.pub_k) >= k;
+      if (__shfl_sync(0xffffffffu, there, 0)) break;
+      if (++polls > kTailSpin) return -1;
+      __nanosleep(20);
+    }
+    __threadfence_block();
+    __syncwarp();
+    a = sm.fac[k % 3];
+    if (tk == 1 || tk >= 3) hits = sm.hit[k % 3];
+  }
+  const int q = lane < n ? lane : 0;
+  const double *g = sm.slot.jvec;
+  double row[9], ug = 0.0;  // row q of U; U^T g, entry q
+#pragma unroll
+  for (int i = 0; i < 9; i++)
+    if (i < n) {
+      row[i] = a[q * n + i];
+      ug += a[i * n + q] * g[i];
+    }
+  double x;
+  if (tk == 1) {
+    double wr = sm.w[q];
+    double wmax = sm.w[0];
+    for (int i = 1; i < n; i++) wmax = fmax(wmax, sm.w[i]);
+    double thr = P.svd_thr;
+    while (true) {
+      const double wthr = wmax * thr;
+      if (wr < wthr) wr = 0.0;
+      const double t = wr > 1e-50 ? ug / wr : 0.0;
+      double tj[9], acc = 0.0;
+#pragma unroll
+      for (int j = 0; j < 9; j++) tj[j] = __shfl_sync(0xffffffffu, t, j);
+#pragma unroll
+      for (int j = 0; j < 9; j++)
+        if (j < n) acc += row[j] * tj[j];
+      x = acc;
+      if (!__any_sync(0xffffffffu, lane < n && (x > 0.5 || x < -0.5))) break;
+      if (thr > 2e-3) {
+        x = x > 0.5 ? 0.5 : (x < -0.5 ? -0.5 : x);
+        break;
+      }
+      thr *= 5.;
+    }
+  } else {
+    x = ug > 0.5 ? 0.5 : (ug < -0.5 ? -0.5 : ug);
+  }
+  // Par_update and bounds_check, lane i for parameter i
+  double v = lane < 9 ? L.par[lane] : 0.0;
+  double dx = 0.0, sx = 0.0;
+  for (int i = 0; i < n; i++) {
+    const double xi = __shfl_sync(0xffffffffu, x, i);
+    if (P.free_idx[i] == lane) {
+      dx = xi;
+      sx = lane == 7 ? L.sc[SC_STEP7] : P.step[lane];
+    }
+  }
+  if (sx != 0.0 || dx != 0.0) v += dx * sx;
+  if (lane == 1 || lane == 2) {
+    const double turn = lane == 1 ? 2.0 * kPi : kPi;
+    double f = fmod(v, turn);
+    if (f < 0) f += turn;
+    if (lane == 1 && f > kPi) f = turn - f;
+    v = f;
+  } else if (lane < 9) {
+    v = clampb(v, lane == 7 ? L.sc[SC_L70] : P.limits[lane][0],
+               lane == 7 ? L.sc[SC_L71] : P.limits[lane][1]);
+  }
+  if (lane < 9) L.ptmp[lane] = v;
+  __syncwarp();
+  return hits;
+}
+
+// jac_store by the first synthesising warp: lane 0 makes the run's set-up and
+// the state, the lanes share the entries.
+template <class T, bool FILT>
+__device__ __forceinline__ void tail_store(const DevPlan &P, TailSmem<T, FILT> &sm, int lane) {
+  TailSlot &o = sm.slot;
+  const int n = P.npar;
+  const double chi0 = sm.hg[54];
+  double ratio = o.sc[SC_RATIO];
+  if (o.state == SL_JAC_START) {
+    ratio = 1.0;
+    if (P.regul_any) {
+      const double pen = penalty_of(P, o.par);
+      if (pen > 0.1 * o.sc[SC_LMCHISQ]) ratio = 0.1 * chi0 / pen;
+    }
+    __syncwarp();
+    if (lane == 0) {
+      o.sc[SC_CHISQ] = chi0;
+      o.sc[SC_RATIO] = ratio;
+      o.it = 0;
+      if (P.niter <= 0) o.state = SL_RUN_END;
+    }
+    if (P.niter <= 0) return;
+  }
+  __syncwarp();
+  for (int e = lane; e < n * n; e += 32) {
+    const int a = e / n, b = e % n;
+    const int ia = P.free_idx[a < b ? a : b], ib = P.free_idx[a < b ? b : a];
+    double h = sm.hg[ia * 9 - ia * (ia + 1) / 2 + ib];
+    if (a == b && P.regul_any && P.regul[ia]) h += P.regul_weight[ia] * ratio;
+    sm.start[e] = h;
+  }
+  if (lane < n) {
+    const int ia = P.free_idx[lane];
+    double gv = sm.hg[45 + ia];
+    if (P.regul_any && P.regul[ia])
+      gv -= (o.par[ia] - P.regul_value[ia]) * P.regul_weight[ia] * ratio;
+    o.jvec[lane] = gv;
+  }
+  if (lane == 0) {
+    o.cnt[1]++;
+    o.sc[SC_DAMP] = P.damp;
+    o.tk = 1;
+    o.state = SL_TRIAL;
+  }
+  __syncwarp();
+}
+
+// Copies slot s of S into the CTA's TailSlot, and its matrix into `start`.
+__device__ __forceinline__ void tail_load(const Slots &S, int s, int n, TailSlot &o,
+                                          double *start, int tid, int threads) {
+  const int W = S.W;
+  if (tid == 0) {
+    o.pix = S.pix[s];
+    o.state = S.state[s];
+    o.run = S.run[s];
+    o.it = S.it[s];
+    o.tk = S.tk[s];
+    o.had_trial = S.had_trial[s];
+  }
+  for (int i = tid; i < 4; i += threads) o.cnt[i] = S.cnt[i * W + s];
+  for (int i = tid; i < SC_COUNT; i += threads) o.sc[i] = S.sc[i * W + s];
+  for (int i = tid; i < 9; i += threads) {
+    o.guess[i] = S.guess[(size_t)i * W + s];
+    o.par[i] = S.par[(size_t)i * W + s];
+    o.pbest[i] = S.pbest[(size_t)i * W + s];
+    o.jvec[i] = S.jvec[(size_t)i * W + s];
+    o.ptmp[i] = S.ptmp[(size_t)i * W + s];
+  }
+  for (int i = tid; i < n * n; i += threads) start[i] = S.hess[(size_t)i * W + s];
+}
+
+}  // namespace detail
+
+template <class T, bool FILT>
+__global__ void __launch_bounds__(TailShape<T, FILT>::kThreads, 1)
+    tail_kernel(const __grid_constant__ DevPlan P, const __grid_constant__ InvertArgs A,
+                  const __grid_constant__ Slots S, int parity, int *cursor) {
+  using Sh = TailShape<T, FILT>;
+  extern __shared__ __align__(16) unsigned char tail_raw[];
+  TailSmem<T, FILT> &sm = *reinterpret_cast<TailSmem<T, FILT> *>(tail_raw);
+  VoigtK<T> K;
+  const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+  if (tid == 0) {
+    TailCtl &c = sm.ctl;
+    c.gen = c.base = c.want = c.quit = c.pub_gen = c.pub_k = c.item = c.error = 0;
+  }
+  voigt_block_setup<T>(K, P, sm.tab);  // (syncs)
+  if (wp == Sh::kSynth) {
+    tail_decompose<T, FILT>(P, sm, lane);
+    return;
+  }
+  T *rden = sm.rden[wp];
+  const int nl = P.nl;
+  const int nj = S.jcount[parity], nr = S.rcount[parity];
+  const long long cap = slot_step_cap(P);
+  Slots L = S;  // the slot in shared memory
+  L.W = 1;
+  L.pix = &sm.slot.pix;
+  L.state = &sm.slot.state;
+  L.run = &sm.slot.run;
+  L.it = &sm.slot.it;
+  L.tk = &sm.slot.tk;
+  L.cnt = sm.slot.cnt;
+  L.had_trial = &sm.slot.had_trial;
+  L.sc = sm.slot.sc;
+  L.guess = sm.slot.guess;
+  L.par = sm.slot.par;
+  L.pbest = sm.slot.pbest;
+  L.jvec = sm.slot.jvec;
+  L.ptmp = sm.slot.ptmp;
+  L.hess = sm.start;
+  Tally t;
+  while (true) {
+    if (tid == 0) sm.ctl.item = atomicAdd(cursor, 1);
+    tail_sync<Sh::kSynth>();
+    const int item = sm.ctl.item;
+    if (item >= nj + nr) break;
+    const int s = item < nj ? S.jlist[parity * S.W + item] : S.rlist[parity * S.W + (item - nj)];
+    tail_load(S, s, P.npar, sm.slot, sm.start, tid, Sh::kPoints);
+    tail_sync<Sh::kSynth>();
+    const double *pp = A.prof + (size_t)sm.slot.pix * 4 * nl;
+    if (sm.slot.state == SL_TRIAL && tid == 0) {
+      // taken up between two trials: the slot's matrix is the factor U_1 for
+      // the second trial, U_(tk - 2) for a later one
+      vstore(&sm.ctl.base, sm.slot.tk <= 2 ? 1 : sm.slot.tk - 2);
+      vstore(&sm.ctl.want, sm.slot.tk);
+      __threadfence_block();
+      vstore(&sm.ctl.gen, sm.ctl.gen + 1);
+    }
+    long long steps = 0;
+    while (true) {
+      tail_sync<Sh::kSynth>();
+      const int st = sm.slot.state;
+      if (st == SL_DONE || st == SL_EMPTY || sm.ctl.error) break;
+      if (++steps > cap) {  // cannot happen for a valid plan
+        tail_sync<Sh::kSynth>();
+        if (tid == 0) sm.ctl.error = 1;
+        continue;
+      }
+      double step[9], sw[4];
+      slot_weights(P, L, 0, step, sw);
+      if (st == SL_JAC_START || st == SL_JAC_NEXT) {
+        double par[9];
+        load9(L.par, 1, 0, par);
+        deriv_tail<T, FILT>(P, K, rden, par, step, pp, sw, tid, sm);
+        if (wp == 0) tail_store<T, FILT>(P, sm, lane);
+        if (tid == 0) {
+          t.jac++;
+          if (sm.slot.state == SL_TRIAL) {
+            vstore(&sm.ctl.base, 0);
+            vstore(&sm.ctl.want, 1);
+            __threadfence_block();
+            vstore(&sm.ctl.gen, sm.ctl.gen + 1);
+          }
+        }
+        continue;
+      }
+      double chi_new = 0.0;
+      if (st == SL_TRIAL) {
+        if (wp == 0) {
+          const int hits = tail_solve<T, FILT>(P, L, sm, lane);
+          if (lane == 0) {
+            if (hits < 0)
+              sm.ctl.error = 1;
+            else
+              t.svdlim += hits;
+          }
+        }
+        tail_sync<Sh::kSynth>();
+        double ptmp[9];
+        load9(L.ptmp, 1, 0, ptmp);
+        chi_new = forward_tail<T, FILT>(P, K, rden, ptmp, step, pp, sw, tid, sm);
+      }
+      if (tid == 0 && !sm.ctl.error) {
+        trial_transition<false>(P, A, L, 0, st, chi_new, 0, t);
+        // rejected: the trial after the next one will want factor tk
+        if (sm.slot.state == SL_TRIAL) vstore(&sm.ctl.want, sm.slot.tk);
+      }
+    }
+    tail_sync<Sh::kSynth>();
+    if (tid == 0 && sm.ctl.error) {  // the pixel ends with a flag
+      if (A.flags) A.flags[sm.slot.pix] = 8;
+      t.busy_delta--;
+      sm.ctl.error = 0;
+    }
+  }
+  if (tid == 0) {
+    vstore(&sm.ctl.quit, 1);
+    t.flush(A, S);
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Lane-split rounds.  Once the queue is empty, the pixels still in flight are
 // too few to fill the GPU one thread each, and every round waits for one
 // thread's synthesis and SVD.  These variants of the round kernels give each
@@ -1338,7 +1976,14 @@ int round_grid_impl(int which, int device) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         &per_sm, trial_kernel<T, FILT, kBlock, false, true>, kBlock, 0);
   } else if (which == 3) {
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, finish_kernel<T, FILT>, kBlock, 0);
+    if constexpr (sizeof(T) == sizeof(float)) {
+      constexpr int smem = (int)sizeof(TailSmem<T, FILT>);
+      cudaFuncSetAttribute(tail_kernel<T, FILT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tail_kernel<T, FILT>,
+                                                    TailShape<T, FILT>::kThreads, smem);
+    } else {
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, finish_kernel<T, FILT>, kBlock, 0);
+    }
   } else {
     cudaFuncSetAttribute(svd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSvdSmem);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, svd_kernel, kSvdBlock, kSvdSmem);
@@ -1498,9 +2143,13 @@ cudaError_t launch_round_grp_impl(int G, const DevPlan &P, const InvertArgs &A, 
 }
 
 template <class T, bool FILT>
-cudaError_t launch_finish_impl(const DevPlan &P, const InvertArgs &A, const Slots &S, int *cursor,
-                               int grid, cudaStream_t st) {
-  finish_kernel<T, FILT><<<grid, kBlock, 0, st>>>(P, A, S, cursor);
+cudaError_t launch_finish_impl(const DevPlan &P, const InvertArgs &A, const Slots &S, int parity,
+                               int *cursor, int grid, cudaStream_t st) {
+  if constexpr (sizeof(T) == sizeof(float))
+    tail_kernel<T, FILT><<<grid, TailShape<T, FILT>::kThreads, sizeof(TailSmem<T, FILT>), st>>>(
+        P, A, S, parity, cursor);
+  else
+    finish_kernel<T, FILT><<<grid, kBlock, 0, st>>>(P, A, S, cursor);
   return cudaGetLastError();
 }
 
@@ -1518,8 +2167,8 @@ cudaError_t launch_finish_impl(const DevPlan &P, const InvertArgs &A, const Slot
     return launch_round_grp_impl<T, FILT>(G, P, A, S, parity, grids, st, ev, ov);                \
   }                                                                                              \
   cudaError_t launch_finish_##SUF(const DevPlan &P, const InvertArgs &A, const Slots &S,         \
-                                  int *cursor, int grid, cudaStream_t st) {                      \
-    return launch_finish_impl<T, FILT>(P, A, S, cursor, grid, st);                               \
+                                  int parity, int *cursor, int grid, cudaStream_t st) {          \
+    return launch_finish_impl<T, FILT>(P, A, S, parity, cursor, grid, st);                       \
   }
 
 }  // namespace me

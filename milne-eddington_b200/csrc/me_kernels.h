@@ -141,11 +141,16 @@ int record_error(int code, const char *msg);
 // CTAs for a full device: which = 0 jac_kernel, 1 trial_kernel, 2 svd_kernel,
 // 3 finish_kernel
 int round_grid(int precision, int which, int device);
-// The tail kernel: runs every slot still in flight to completion, one warp
-// per slot (slots taken through *cursor, zeroed by the caller).  Only when the
-// queue is exhausted (it does not refill).
+// The tail kernel: runs every slot still in flight (FP32: those on the lists of
+// the round `parity`) to completion, one CTA (FP32) or one warp (FP64) per slot
+// (taken through *cursor, zeroed by the caller).  Only when the queue is
+// exhausted (it does not refill).
+inline int finish_pixels(int precision) { return precision == 1 ? kBlock / 32 : 1; }
 cudaError_t launch_finish(int precision, const DevPlan &P, const InvertArgs &A, const Slots &S,
-                          int *cursor, int grid, cudaStream_t st);
+                          int parity, int *cursor, int grid, cudaStream_t st);
+// Pixels in flight per SM at or below which, with the queue empty, the tail
+// kernel takes over by default.
+constexpr int kTailPerSm = 4;
 // One round: jac_kernel, svd (first trials), svd (later trials),
 // trial_kernel.  grids: jac, trial, svd CTAs.  ev (nullable): 5 events
 // recorded before, between and after the four launches (per-kernel device

@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(256) order_scatter_kernel(const unsigned char 
                                      const Slots &S, int parity, const int grids[3],             \
                                      cudaStream_t st, cudaEvent_t *ev, const Overlap *ov);       \
   cudaError_t launch_finish_##SUF(const DevPlan &P, const InvertArgs &A, const Slots &S,         \
-                                  int *cursor, int grid, cudaStream_t st);
+                                  int parity, int *cursor, int grid, cudaStream_t st);
 ME_DECLARE_ROUNDS(f32)
 ME_DECLARE_ROUNDS(f64)
 ME_DECLARE_ROUNDS(f32f)
@@ -300,8 +300,8 @@ ME_DECLARE_ROUNDS(f64f)
                   : (P.nsub > 1 ? FN##_f32f(__VA_ARGS__) : FN##_f32(__VA_ARGS__)))
 
 cudaError_t launch_finish(int precision, const DevPlan &P, const InvertArgs &A, const Slots &S,
-                          int *cursor, int grid, cudaStream_t st) {
-  return ME_PICK(launch_finish, P, A, S, cursor, grid, st);
+                          int parity, int *cursor, int grid, cudaStream_t st) {
+  return ME_PICK(launch_finish, P, A, S, parity, cursor, grid, st);
 }
 
 cudaError_t launch_round_grp(int precision, int G, const DevPlan &P, const InvertArgs &A,
@@ -316,11 +316,11 @@ cudaError_t launch_round_grp(int precision, int G, const DevPlan &P, const Inver
 // the SVD grid raises that limit, so it is done in the filtered unit of the
 // precision too (a plan may take a filter after it is made).
 int round_grid(int precision, int which, int device) {
-  if (which == 2) {
+  if (which == 2 || which == 3) {
     if (precision == 1)
-      round_grid_f64f(2, device);
+      round_grid_f64f(which, device);
     else
-      round_grid_f32f(2, device);
+      round_grid_f32f(which, device);
   }
   return precision == 1 ? round_grid_f64(which, device) : round_grid_f32(which, device);
 }
