@@ -16,74 +16,147 @@ namespace {
 // Building blocks exposed for the unit entry points.
 // ---------------------------------------------------------------------------
 
+
+// Syntheses of npix parameter sets (and, JAC, their Jacobians).  A block takes
+// `per` pixels: its first threads set them up (the terms that do not depend
+// on the wavelength) in shared memory, then all its threads take points
+// (pixel, wavelength) in the order of the output, so that stores run along the
+// wavelengths.  One thread per pixel stored 8 bytes every 32 nl (288 nl with
+// the Jacobian) and left most of the device idle on maps of a few thousand
+// pixels.
+// flags (nullable): pixels without bit 0 get zeros instead.
+// Measured on a B200, one thread per pixel against this: 262144 profiles of 60
+// wavelengths, FP32, 912 -> 288 us; 10007 FP64 Jacobians of 112 wavelengths 1600
+// -> 533 us; 37 FP32 Jacobians 147 -> 20 us (host call included).  The large FP32
+// map is bound by instruction issue (0.87 per cycle and scheduler).
+constexpr int kSynthThreads = 128;
 template <class T>
-__global__ void synth_kernel(const DevPlan P, const double *par, long long npix, double step7,
-                             double *prof, double *jac) {
-  __shared__ T s_tab[100];
-  __shared__ T s_rden[kRden * 128];
-  VoigtK<T> K;
-  voigt_block_setup<T>(K, P, s_tab);
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= npix) return;
-  const int nl = P.nl;
-  double step[9];
-#pragma unroll
-  for (int k = 0; k < 9; k++) step[k] = P.step[k];
-  step[7] = step7;
-  double mp[9];
-#pragma unroll
-  for (int k = 0; k < 9; k++) mp[k] = par[i * 9 + k];
-  SynthCall<T> c;
-  synth_setup<T>(c, mp, P, step);
-  voigt_prepare<T>(K, c.p5, s_rden + threadIdx.x, blockDim.x);
-  const T ones[4] = {T(1), T(1), T(1), T(1)};
-  for (int iw = 0; iw < nl; iw++) {
-    T syn[4], J[4][9];
-    if (jac) {
-      if (P.nsub > 1)
-        channel_point<T, true, true>(c, P, K, ones, iw, syn, J);
-      else
-        channel_point<T, true, false>(c, P, K, ones, iw, syn, J);
-      for (int s = 0; s < 4; s++)
-        for (int k = 0; k < 9; k++) jac[((size_t)i * 36 + s * 9 + k) * nl + iw] = (double)J[s][k];
-    } else if (P.nsub > 1) {
-      channel_point<T, false, true>(c, P, K, ones, iw, syn, nullptr);
-    } else {
-      channel_point<T, false, false>(c, P, K, ones, iw, syn, nullptr);
-    }
-    for (int s = 0; s < 4; s++) prof[((size_t)i * 4 + s) * nl + iw] = (double)syn[s];
-  }
-}
+constexpr int kSynthPixels = sizeof(T) == sizeof(float) ? 32 : 16;  // most per block
 
 template <class T>
-__global__ void fit_kernel(const DevPlan P, const double *fitpar, const unsigned char *flags,
-                           long long npix, double *fit) {
+struct SynthPixel {
+  SynthCall<T> c;
+  T yy, inv_y;
+  T rden[sizeof(T) == sizeof(float) ? kRden : 1];
+};
+
+enum SynthMode { kPlain, kFilter, kFilterSplit };  // no filter; with one: see launch_synth_t
+
+template <class T, bool JAC, int MODE>
+__global__ void __launch_bounds__(kSynthThreads)
+    synth_kernel(const __grid_constant__ DevPlan P, const double *par, const unsigned char *flags,
+                 long long npix, int per, double step7, double *prof, double *jac) {
   __shared__ T s_tab[100];
-  __shared__ T s_rden[kRden * 128];
+  __shared__ SynthPixel<T> s_px[kSynthPixels<T>];
   VoigtK<T> K;
   voigt_block_setup<T>(K, P, s_tab);
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= npix) return;
+  const long long first = blockIdx.x * (long long)per;
+  const int here = (int)(npix - first < per ? npix - first : per);
+  if ((int)threadIdx.x < here) {
+    SynthPixel<T> &o = s_px[threadIdx.x];
+    const long long i = first + threadIdx.x;
+    double mp[9], step[9];
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+      mp[k] = par[i * 9 + k];
+      step[k] = P.step[k];
+    }
+    step[7] = step7;
+    SynthCall<T> c;
+    synth_setup<T>(c, mp, P, step);
+    voigt_prepare<T>(K, c.p5, o.rden, 1);
+    o.c = c;
+    o.yy = K.yy;
+    o.inv_y = K.inv_y;
+  }
+  __syncthreads();
   const int nl = P.nl;
-  double *out = fit + (size_t)i * 4 * nl;
-  if (!(flags[i] & 1)) {
-    for (int k = 0; k < 4 * nl; k++) out[k] = 0.0;
+  const T ones[4] = {T(1), T(1), T(1), T(1)};
+  K.rstride = 1;
+  if constexpr (MODE == kFilterSplit) {
+    // a point is a sub-wavelength; entry e of an observed value (the profiles,
+    // then the Jacobian's J[s][k]) is summed over its sub-wavelengths in
+    // order, from zero, by one thread (part: its sum so far, when the points of
+    // a wavelength straddle two batches)
+    constexpr int E = JAC ? 40 : 4;
+    __shared__ T s_pt[kSynthThreads * E];
+    __shared__ T s_part[E];
+    const int ns = P.nsub, tid = threadIdx.x, total = here * nl * ns;
+    for (int p0 = 0; p0 < total; p0 += kSynthThreads) {
+      const int e = p0 + tid;
+      if (e < total) {
+        const int p = e / (nl * ns);
+        const SynthPixel<T> &o = s_px[p];
+        K.yy = o.yy;
+        K.inv_y = o.inv_y;
+        K.rden = o.rden;
+        T ys[4], Jq[4][9];
+        me_point<T, JAC>(o.c, shift_wf<T>(o.c, P, e - p * nl * ns), K, ones, ys,
+                         JAC ? Jq : nullptr);
+#pragma unroll
+        for (int s = 0; s < 4; s++) s_pt[tid * E + s] = ys[s];
+        if (JAC) {
+#pragma unroll
+          for (int s = 0; s < 4; s++)
+#pragma unroll
+            for (int k = 0; k < 9; k++) s_pt[tid * E + 4 + s * 9 + k] = Jq[s][k];
+        }
+      }
+      __syncthreads();
+      const int p1 = p0 + kSynthThreads < total ? p0 + kSynthThreads : total;
+      const int w0 = p0 / ns, w1 = (p1 - 1) / ns;
+      T carry = T(0);
+      for (int u = tid; u < (w1 - w0 + 1) * E; u += kSynthThreads) {
+        const int w = w0 + u / E, m = u % E;
+        const int q0 = w * ns > p0 ? w * ns : p0;
+        const int q1 = (w + 1) * ns < p1 ? (w + 1) * ns : p1;
+        T v = q0 == w * ns ? T(0) : s_part[m];
+        for (int q = q0; q < q1; q++) v += T(P.sub_w[q - w * ns]) * s_pt[(q - p0) * E + m];
+        if (q1 < (w + 1) * ns) {
+          carry = v;
+          continue;
+        }
+        const size_t i = (size_t)(first + w / nl);
+        const int iw = w % nl;
+        const bool live = !flags || (flags[i] & 1);
+        if (m < 4)
+          prof[(i * 4 + m) * nl + iw] = live ? (double)v : 0.0;
+        else
+          jac[(i * 36 + m - 4) * nl + iw] = (double)v;
+      }
+      __syncthreads();
+      if (p1 < (w1 + 1) * ns) {
+        for (int u = tid; u < (w1 - w0 + 1) * E; u += kSynthThreads)
+          if (u / E == w1 - w0) s_part[u % E] = carry;
+        __syncthreads();
+      }
+    }
     return;
   }
-  double mp[9];
+  for (int e = threadIdx.x; e < here * nl; e += kSynthThreads) {
+    const int p = e / nl, iw = e - p * nl;
+    const SynthPixel<T> &o = s_px[p];
+    const size_t i = (size_t)(first + p);
+    double *out = prof + i * 4 * nl + iw;
+    if (flags && !(flags[i] & 1)) {
 #pragma unroll
-  for (int k = 0; k < 9; k++) mp[k] = fitpar[i * 9 + k];
-  SynthCall<T> c;
-  synth_setup<T>(c, mp, P, P.step);
-  voigt_prepare<T>(K, c.p5, s_rden + threadIdx.x, blockDim.x);
-  const T ones[4] = {T(1), T(1), T(1), T(1)};
-  for (int iw = 0; iw < nl; iw++) {
-    T syn[4];
-    if (P.nsub > 1)
-      channel_point<T, false, true>(c, P, K, ones, iw, syn, nullptr);
-    else
-      channel_point<T, false, false>(c, P, K, ones, iw, syn, nullptr);
-    for (int s = 0; s < 4; s++) out[s * nl + iw] = (double)syn[s];
+      for (int s = 0; s < 4; s++) out[s * nl] = 0.0;
+      continue;
+    }
+    K.yy = o.yy;
+    K.inv_y = o.inv_y;
+    K.rden = o.rden;
+    T syn[4], J[4][9];
+    channel_point<T, JAC, MODE == kFilter>(o.c, P, K, ones, iw, syn, JAC ? J : nullptr);
+#pragma unroll
+    for (int s = 0; s < 4; s++) out[s * nl] = (double)syn[s];
+    if (JAC) {
+      double *jo = jac + i * 36 * nl + iw;
+#pragma unroll
+      for (int s = 0; s < 4; s++)
+#pragma unroll
+        for (int k = 0; k < 9; k++) jo[(s * 9 + k) * nl] = (double)J[s][k];
+    }
   }
 }
 
@@ -331,28 +404,71 @@ cudaError_t launch_round(int precision, const DevPlan &P, const InvertArgs &A, c
   return ME_PICK(launch_round, P, A, S, parity, grids, st, ev, svd_lanes, ov);
 }
 
+template <class T>
+static void launch_synth_t(const DevPlan &P, const double *d_par, const unsigned char *d_flags,
+                           long long npix, double step7, double *d_prof, double *d_jac,
+                           cudaStream_t st) {
+  // pixels per block: up to kSynthPixels, fewer while the grid has less than
+  // four blocks per SM, so that a few pixels spread over the device; of the
+  // upper half of that range, the count whose wavelengths leave the fewest of
+  // the block's threads idle in its last pass (6 wavelengths: 21 pixels)
+  constexpr long long kBlocks = 148 * 4;
+  int per = kSynthPixels<T>;
+  while (per > 1 && (npix + per - 1) / per < kBlocks) per /= 2;
+  auto used = [&](int n) {
+    const int points = n * P.nl;
+    return (double)points / ((points + kSynthThreads - 1) / kSynthThreads * kSynthThreads);
+  };
+  if (per == kSynthPixels<T>)
+    for (int n = per - 1; n >= per / 2; n--)
+      if (used(n) > used(per) + 0.05) per = n;
+  const unsigned g = (unsigned)((npix + per - 1) / per);
+  // with a filter a point is a sub-wavelength, its terms staged in shared
+  // memory; with enough wavelengths to fill the device a thread sums its
+  // wavelength's sub-wavelengths itself, which stages nothing (Fe I 6173, 21
+  // sub-wavelengths, FP32: 48087 pixels 121 us against 180, 32 pixels 32 us
+  // against 18).  FP64 Jacobians are always split: 40 sums of doubles beside
+  // the point's registers spill (17486 pixels 1231 us against 906)
+  const int mode = P.nsub <= 1 ? kPlain
+                   : npix * P.nl >= 148 * (d_jac ? 512 : 1024) ? kFilter : kFilterSplit;
+  auto go = [&](auto jac, auto m) {
+    synth_kernel<T, jac.value, m.value><<<g, kSynthThreads, 0, st>>>(
+        P, d_par, d_flags, npix, per, step7, d_prof, d_jac);
+  };
+  auto pick = [&](auto jac) {
+    if (mode == kPlain)
+      go(jac, std::integral_constant<int, kPlain>());
+    else if constexpr (jac.value && sizeof(T) == sizeof(double))
+      go(jac, std::integral_constant<int, kFilterSplit>());
+    else if (mode == kFilter)
+      go(jac, std::integral_constant<int, kFilter>());
+    else
+      go(jac, std::integral_constant<int, kFilterSplit>());
+  };
+  if (d_jac)
+    pick(std::true_type());
+  else
+    pick(std::false_type());
+}
+
 cudaError_t launch_synth(int precision, const DevPlan &P, const double *d_par, long long npix,
                          double step7, double *d_prof, double *d_jac, cudaStream_t st) {
-  const int b = 128;
-  const unsigned g = (unsigned)((npix + b - 1) / b);
-  if (g == 0) return cudaSuccess;
+  if (npix <= 0) return cudaSuccess;
   if (precision == 1)
-    synth_kernel<double><<<g, b, 0, st>>>(P, d_par, npix, step7, d_prof, d_jac);
+    launch_synth_t<double>(P, d_par, nullptr, npix, step7, d_prof, d_jac, st);
   else
-    synth_kernel<float><<<g, b, 0, st>>>(P, d_par, npix, step7, d_prof, d_jac);
+    launch_synth_t<float>(P, d_par, nullptr, npix, step7, d_prof, d_jac, st);
   return cudaGetLastError();
 }
 
 cudaError_t launch_fit(int precision, const DevPlan &P, const double *d_fitpar,
                        const unsigned char *d_flags, long long npix, double *d_fit,
                        cudaStream_t st) {
-  const int b = 128;
-  const unsigned g = (unsigned)((npix + b - 1) / b);
-  if (g == 0) return cudaSuccess;
+  if (npix <= 0) return cudaSuccess;
   if (precision == 1)
-    fit_kernel<double><<<g, b, 0, st>>>(P, d_fitpar, d_flags, npix, d_fit);
+    launch_synth_t<double>(P, d_fitpar, d_flags, npix, P.step[7], d_fit, nullptr, st);
   else
-    fit_kernel<float><<<g, b, 0, st>>>(P, d_fitpar, d_flags, npix, d_fit);
+    launch_synth_t<float>(P, d_fitpar, d_flags, npix, P.step[7], d_fit, nullptr, st);
   return cudaGetLastError();
 }
 
