@@ -1679,8 +1679,7 @@ static __device__ __noinline__ void svd9_cancel(double *t, int rows, double *w, 
 // left unrotated.
 constexpr int kSvd9Words = 9 + 9 + 16;  // doubles of shared memory per thread: w, rv1, cs
 
-// The Householder reduction and the accumulation of the left-hand
-// transformations into A; returns anorm.
+// The Householder reduction of A to bidiagonal form (w, rv1); returns anorm.
 template <int STR>
 __device__ __forceinline__ double svd9_reduce(double (&A)[9][9], double *w, double *rv1) {
   constexpr int n = 9, m = 9;
@@ -1755,7 +1754,14 @@ __device__ __forceinline__ double svd9_reduce(double (&A)[9][9], double *w, doub
     const double t = __dadd_rn(fabs(wi), fabs(rvi));
     if (anorm < t) anorm = t;
   }
-  // accumulation of the left-hand transformations into U
+  return anorm;
+}
+
+// The accumulation of the left-hand transformations into A.  DIVIDE: gr_svd's
+// form (s / a_ii) g, where gr_svd_u has s (1 / a_ii) g.
+template <int STR, bool DIVIDE = false>
+__device__ __forceinline__ void svd9_left(double (&A)[9][9], const double *w) {
+  constexpr int n = 9, m = 9;
 #pragma unroll
   for (int i = n - 1; i >= 0; i--) {
     const int l = i + 1;
@@ -1770,7 +1776,8 @@ __device__ __forceinline__ double svd9_reduce(double (&A)[9][9], double *w, doub
         double sj = 0.0;
 #pragma unroll
         for (int k = l; k < m; k++) sj = __fma_rn(A[k][i], A[k][j], sj);
-        const double fj = __dmul_rn(__dmul_rn(sj, iaii), gi);
+        const double fj =
+            __dmul_rn(DIVIDE ? sj / A[i][i] : __dmul_rn(sj, iaii), gi);
 #pragma unroll
         for (int k = i; k < m; k++) A[k][j] = __fma_rn(fj, A[k][i], A[k][j]);
       }
@@ -1782,15 +1789,22 @@ __device__ __forceinline__ double svd9_reduce(double (&A)[9][9], double *w, doub
     }
     A[i][i] = __dadd_rn(A[i][i], 1.0);
   }
-  return anorm;
 }
 
-// The implicit-shift QR sweeps, applied to R rows of U in Q.  stop() is asked
+// What the sweeps do to V: nothing here (V = U in the trial steps' solves).
+struct NoRight {
+  __device__ __forceinline__ void record(int, double, double) {}
+  __device__ __forceinline__ void apply(int, int) {}
+  __device__ __forceinline__ void negate(int) {}
+};
+
+// The implicit-shift QR sweeps, applied to R rows of U in Q (and, by `right`, to
+// V).  stop() is asked
 // before each sweep; the sweeps are left when it says so.  Returns 1 when a
 // singular value needed more than 50 sweeps.
-template <int FORM, bool FAST, int STR, int R, class Stop>
+template <int FORM, bool FAST, int STR, int R, class Stop, class Right = NoRight>
 __device__ __forceinline__ int svd9_sweeps(double (&Q)[R][9], double *w, double *rv1, double *cs,
-                                           double anorm, Stop stop) {
+                                           double anorm, Stop stop, Right right = Right()) {
   constexpr int n = 9;
   int hit = 0;
   int k = n - 1, its = 0;
@@ -1810,7 +1824,10 @@ __device__ __forceinline__ int svd9_sweeps(double (&Q)[R][9], double *w, double 
       l = z ? 31 - __clz(z) : 0;
       cancel = z && !((zr >> l) & 1u);
       if (cancel || l != k) break;
-      if (w[k * STR] < 0.0) w[k * STR] = -w[k * STR];
+      if (w[k * STR] < 0.0) {
+        w[k * STR] = -w[k * STR];
+        right.negate(k);
+      }
       its = 0;
       if (--k < 0) break;
     }
@@ -1827,7 +1844,10 @@ __device__ __forceinline__ int svd9_sweeps(double (&Q)[R][9], double *w, double 
 #pragma unroll
         for (int c = 0; c < n; c++) Q[r][c] = t[r * 9 + c];
       if (l == k) {
-        if (w[k * STR] < 0.0) w[k * STR] = -w[k * STR];
+        if (w[k * STR] < 0.0) {
+          w[k * STR] = -w[k * STR];
+          right.negate(k);
+        }
         its = 0;
         k--;
         continue;
@@ -1875,6 +1895,7 @@ __device__ __forceinline__ int svd9_sweeps(double (&Q)[R][9], double *w, double 
           c = f / z;
           s = h / z;
         }
+        right.record(j, c, s);
         rv1[j * STR] = z;
         f = __fma_rn(x, c, __dmul_rn(g1, s));
         g1 = __fma_rn(g1, c, -__dmul_rn(x, s));
@@ -1902,6 +1923,7 @@ __device__ __forceinline__ int svd9_sweeps(double (&Q)[R][9], double *w, double 
       {
         double h = __dmul_rn(s, g0), g1 = __dmul_rn(g0, c), y = y0;
         double z = radius9<FORM, FAST, false>(f, h, c, s);
+        right.record(j, c, s);
         rv1[j * STR] = z;
         f = __fma_rn(x, c, __dmul_rn(g1, s));
         g1 = __fma_rn(g1, c, -__dmul_rn(x, s));
@@ -1919,6 +1941,7 @@ __device__ __forceinline__ int svd9_sweeps(double (&Q)[R][9], double *w, double 
     rv1[l * STR] = 0.0;
     rv1[k * STR] = f;
     w[k * STR] = x;
+    right.apply(l, k);
     // its rotations, on columns j and j + 1 of A
     double nc = cs[0], ns = cs[STR];
 #pragma unroll
@@ -1952,7 +1975,78 @@ struct NeverStop {
 template <int FORM, bool FAST, int STR>
 __device__ __forceinline__ int gr_svd9(double (&A)[9][9], double *w, double *rv1, double *cs) {
   const double anorm = svd9_reduce<STR>(A, w, rv1);
+  svd9_left<STR>(A, w);
   return svd9_sweeps<FORM, FAST, STR, 9>(A, w, rv1, cs, anorm, NeverStop());
+}
+
+// V of gr_svd9_v in shared memory, one thread's 81 elements from v on (row-major):
+// the right-hand rotations of a sweep are recorded in cv and applied after its
+// chain, column by column, with the shared column carried in registers.
+template <int STR>
+struct RightInShared {
+  double *v, *cv;
+  __device__ __forceinline__ void record(int j, double c, double s) {
+    cv[j * 2 * STR] = c;
+    cv[(j * 2 + 1) * STR] = s;
+  }
+  __device__ __forceinline__ void apply(int l, int k) {
+    double x[9];
+#pragma unroll
+    for (int r = 0; r < 9; r++) x[r] = v[r * 9 + l];
+#pragma unroll 1
+    for (int j = l; j < k; j++) {
+      const double c = cv[j * 2 * STR], s = cv[(j * 2 + 1) * STR];
+#pragma unroll
+      for (int r = 0; r < 9; r++) {
+        const double z = v[r * 9 + j + 1];
+        v[r * 9 + j] = __fma_rn(x[r], c, __dmul_rn(z, s));
+        x[r] = __fma_rn(z, c, -__dmul_rn(x[r], s));
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 9; r++) v[r * 9 + k] = x[r];
+  }
+  __device__ __forceinline__ void negate(int k) {
+    for (int r = 0; r < 9; r++) v[r * 9 + k] = -v[r * 9 + k];
+  }
+};
+
+static __device__ __noinline__ double divide_d(double a, double b) { return a / b; }
+
+// gr_svd for a 9 x 9 matrix, one thread per matrix: gr_svd9 with V.  A in
+// registers; v: 81 doubles of shared memory of this thread's own, row-major.
+// The right-hand transformations are accumulated into V from A's rows before
+// the left-hand ones overwrite them.
+template <int STR>
+__device__ __forceinline__ int gr_svd9_v(double (&A)[9][9], double *w, double *rv1, double *cs,
+                                         double *cv, double *v) {
+  constexpr int n = 9;
+  const double anorm = svd9_reduce<STR>(A, w, rv1);
+#pragma unroll
+  for (int i = n - 1; i >= 0; i--) {
+    const int l = i + 1;
+    if (i < n - 1) {
+      const double g = rv1[l * STR];
+      if (g != 0.0) {
+#pragma unroll
+        for (int j = l; j < n; j++) v[j * 9 + i] = divide_d(divide_d(A[i][j], A[i][l]), g);
+#pragma unroll 1
+        for (int j = l; j < n; j++) {
+          double s = 0.0;
+#pragma unroll
+          for (int k = l; k < n; k++) s = __fma_rn(A[i][k], v[k * 9 + j], s);
+#pragma unroll
+          for (int k = l; k < n; k++) v[k * 9 + j] = __fma_rn(s, v[k * 9 + i], v[k * 9 + j]);
+        }
+      }
+#pragma unroll
+      for (int j = l; j < n; j++) v[i * 9 + j] = v[j * 9 + i] = 0.0;
+    }
+    v[i * 9 + i] = 1.0;
+  }
+  svd9_left<STR, true>(A, w);
+  return svd9_sweeps<0, false, STR, 9>(A, w, rv1, cs, anorm, NeverStop(),
+                                       RightInShared<STR>{v, cv});
 }
 
 // gr_svd9 of one matrix by a warp, for the least latency: every lane reduces
@@ -1971,6 +2065,7 @@ __device__ __forceinline__ int gr_svd9_warp(const double *a, double *u, double *
 #pragma unroll
       for (int c = 0; c < 9; c++) A[r][c] = a[r * 9 + c];
     anorm = svd9_reduce<STR>(A, w, rv1);
+    svd9_left<STR>(A, w);
 #pragma unroll
     for (int c = 0; c < 9; c++) {
       q[0][c] = A[0][c];
@@ -1999,12 +2094,6 @@ __device__ __forceinline__ int gr_svd9_warp(const double *a, double *u, double *
 // changes.  w [n] is private to the lane.  All lanes of the group call it.
 template <int G, bool FAST = false>
 __device__ __noinline__ int gr_svd_u_grp(double *a, int n, double *w, int lane, unsigned mask) {
-  if constexpr (G == 32) {
-    if (n == 9) {  // the same bits in less time
-      double rv1[9], cs[16];
-      return gr_svd9_warp<1, FAST, 1>(a, a, w, rv1, cs, lane, NeverStop());
-    }
-  }
 #define A_(i, j) a[(i) * n + (j)]
 #define GSYNC()                  \
   do {                           \
@@ -2231,6 +2320,20 @@ __device__ __noinline__ int gr_svd_u_grp(double *a, int n, double *w, int lane, 
 #undef FOR9
 #undef GSYNC
 #undef A_
+}
+
+// gr_svd_u_grp by a whole warp; order 9 through gr_svd9_warp, which gives the
+// same bits in less time (functions of their own: the compiler's contraction
+// of each depends on all that is inlined in it).
+template <bool FAST>
+static __device__ __noinline__ int gr_svd9_alone(double *a, double *w, int lane) {
+  double rv1[9], cs[16];
+  return gr_svd9_warp<1, FAST, 1>(a, a, w, rv1, cs, lane, NeverStop());
+}
+template <bool FAST>
+static __device__ __noinline__ int gr_svd_u_warp(double *a, int n, double *w, int lane) {
+  if (n == 9) return gr_svd9_alone<FAST>(a, w, lane);
+  return gr_svd_u_grp<32, FAST>(a, n, w, lane, 0xffffffffu);
 }
 
 // x = V diag(1/w) U^T b, skipping w <= 1e-50 (svbksb, SVD_TEMPLATE.h:348-406).

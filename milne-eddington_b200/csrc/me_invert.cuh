@@ -450,7 +450,9 @@ __device__ __forceinline__ int solve_slot(const DevPlan &P, const Slots &S, int 
   for (int k = WARP ? lane : 0; k < n * n; k += G) a[k * STR] = S.hess[(size_t)k * W + s];
   if (WARP) __syncwarp(mask);
   auto decompose = [&]() {
-    if constexpr (WARP)
+    if constexpr (G == 32)
+      return P.fastg ? gr_svd_u_warp<true>(a, n, w, lane) : gr_svd_u_warp<false>(a, n, w, lane);
+    else if constexpr (WARP)
       return P.fastg ? gr_svd_u_grp<G, true>(a, n, w, lane, mask)
                      : gr_svd_u_grp<G, false>(a, n, w, lane, mask);
     else

@@ -75,3 +75,22 @@ def _check(a, lanes, fast):
 def test_zero_matrix():
     u, w, hits = me_b200.svd_u(np.zeros((3, 9, 9)))
     assert hits == 0 and np.all(w == 0) and np.all(u == np.eye(9))
+
+
+@pytest.mark.parametrize("count", [1, 33, 1185, 20011])
+@pytest.mark.parametrize("kind", ["normal", "rank4", "orthogonal", "zero_pivot"])
+def test_full_decomposition(kind, count):
+    """me_svd at order 9 (gr_svd9_v): a = u diag(w) v^T, u and v orthogonal
+    where w is not zero, to the bounds above."""
+    a = _inputs(kind, count)
+    u, w, v = me_b200.svd(a)
+    scale = np.linalg.norm(a, axis=(1, 2))[:, None]
+    unit, ws = a / scale[:, :, None], w / scale
+    assert np.all(w >= 0)
+    assert np.max(np.abs(np.einsum("mik,mk,mjk->mij", u, ws, v) - unit)) < 1e-12
+    eye = np.einsum("mki,mkj->mij", v, v)
+    assert np.max(np.abs(eye - np.eye(9))) < 1e-13
+    live = ws > 1e-13
+    both = live[:, :, None] & live[:, None, :]
+    eye = np.einsum("mki,mkj->mij", u, u)
+    assert np.max(np.abs(np.where(both, eye - np.eye(9), 0.0))) < 1e-13
