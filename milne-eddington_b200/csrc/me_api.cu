@@ -1082,9 +1082,7 @@ int invert_impl(me_plan *p, const double *d_prof, long npix, double *d_res, doub
     stats->wavelengths = (long long)(tot[3] + tot[5]) * p->P.nl;
     stats->redo_pixels = redo_total;
     stats->launches = 4 * rounds_total + p->finish_launches + (d_fit ? 1 : 0) +
-                      (p->init ? me::kMlpPredLaunches *
-                                     ((npix + me::kMlpPredChunk - 1) / me::kMlpPredChunk)
-                               : 0);
+                      (p->init ? me::mlp_predict_launches(p->init, npix) : 0);
     stats->rounds = rounds_total;
     stats->kernel_ms = kernel_ms;
     stats->init_ms = init_ms;

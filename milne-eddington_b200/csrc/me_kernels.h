@@ -36,12 +36,15 @@ inline int svd_grid(int npar, int wave, int W) {
   const int need = (W + per - 1) / per;
   return need < wave ? need : wave;
 }
-// learned initialiser inference: rows per chunk, kernel launches per chunk
+// learned initialiser inference with the mma.sync GEMMs: rows per chunk, kernel
+// launches per chunk
 constexpr int kMlpPredChunk = 65536;
 constexpr int kMlpPredLaunches = 6;
 // error status of the initialiser's tensor-core GEMMs since the last call
 // (a bounded wait that expired); synchronises the device (me_mlp.cu)
 int mlp_gemm_status(me_mlp *m);
+// kernels that the inference of npix profiles launches
+long long mlp_predict_launches(const me_mlp *m, long long npix);
 
 // Life cycle of an inversion slot (one pixel in flight).
 enum SlotStateCode : int {

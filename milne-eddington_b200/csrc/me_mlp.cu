@@ -384,8 +384,10 @@ bool cached_tile_map(TileMapCache *c, CUtensorMap *map, const bf16 *p, int rows,
 // and whether the kernel's shared-memory limit has been raised.
 struct DeviceFacts {
   int sms = 0;
-  bool smem_ok = false;
+  bool smem_ok = false, pred_ok = false;
 };
+
+bool predict_kernel_ready();  // (below, with the kernel)
 
 const DeviceFacts &device_facts() {
   static DeviceFacts facts[64];
@@ -401,6 +403,7 @@ const DeviceFacts &device_facts() {
       f.sms = 0;
     f.smem_ok = cudaFuncSetAttribute(umma_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      me::umma::kSmemMax) == cudaSuccess;
+    f.pred_ok = predict_kernel_ready();
     facts[dev] = f;
   });
   return facts[dev];
@@ -637,15 +640,12 @@ __global__ void __launch_bounds__(256)
   if (lane == 0) imax_out[i] = (float)imax;
 }
 
-// network outputs (standardised) -> the nine ME parameters [n][9] (FP64)
-__global__ void decode_kernel(const float *Y, long long n, int ld, const float *tmean,
-                              const float *tstd, const float *imax, double *par) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
+// network outputs (standardised, one row y) -> the nine ME parameters p[9] (FP64)
+__device__ __forceinline__ void decode_row(const float *y, const float *tmean, const float *tstd,
+                                           float imax, double *p) {
   float t[kOut];
 #pragma unroll
-  for (int k = 0; k < kOut; k++) t[k] = Y[(size_t)i * ld + k] * tstd[k] + tmean[k];
-  double *p = par + (size_t)i * 9;
+  for (int k = 0; k < kOut; k++) t[k] = y[k] * tstd[k] + tmean[k];
   p[0] = fmax((double)t[0], 0.0);
   p[1] = acos(fmin(fmax((double)t[1], -1.0), 1.0));
   double phi = 0.5 * atan2((double)t[2], (double)t[3]);
@@ -655,8 +655,340 @@ __global__ void decode_kernel(const float *Y, long long n, int ld, const float *
   p[4] = t[5];
   p[5] = t[6];
   p[6] = t[7];
-  p[7] = (double)t[9] * imax[i];
+  p[7] = (double)t[9] * imax;
   p[8] = t[8];
+}
+
+__global__ void decode_kernel(const float *Y, long long n, int ld, const float *tmean,
+                              const float *tstd, const float *imax, double *par) {
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  decode_row(Y + (size_t)i * ld, tmean, tstd, imax[i], par + (size_t)i * 9);
+}
+
+// ---------------------------------------------------------------------------
+// The whole inference of a map in one kernel: features, the four layers on the
+// tensor cores, the decode.  A CTA holds two tiles of 128 profiles, each with
+// eight working warps, which write the features, and after each layer the
+// activations, as BF16 into the tile the next layer reads (K-major, 128-byte
+// swizzle).  One more warp brings the weights in (TMA, 64 inputs of a layer per
+// stage) and one issues the MMAs into each tile's 256 FP32 tensor-memory
+// columns, for one tile while the other is in its epilogue: with the loads on
+// the issuing lane, and half of N per instruction, a layer's MMAs took 7,100
+// cycles, as they are 2,500.  Rows of more than 256 features go through the
+// first layer in pieces of 256.  Nothing of a profile's activations leaves the
+// SM.  The epilogues bound it, by their instructions: some 45 per GELU (erff,
+// as in the separate kernels: its results are rounded to BF16, and another form
+// would turn some of them), 69 of the 97 thousand cycles of a pair of tiles;
+// the features take another 12, with the next pair's profiles asked into L2
+// ahead of time (before that, and with a row's loads in pairs only, 40).
+// The values are those of map_features_kernel, umma_gemm_kernel and
+// decode_kernel, which did this in six launches with every layer's activations
+// through memory.  Profiles of 60 wavelengths, there and here, us:
+//   1: 46, 45;  1,000: 53, 47;  18,900: 90, 50;  37,889: 162, 95;  300,007: 921, 493
+// and of 112: 1: 52, 51;  18,900: 106, 56;  75,000: 313, 163.  So it is used at
+// every count; the six launches remain for the mma.sync GEMMs.
+// Waits are bounded as in umma_gemm_kernel; after one runs out the CTA writes a
+// code to *err, stops loading and multiplying, keeps its barriers in step and
+// leaves its results unwritten.
+// ---------------------------------------------------------------------------
+constexpr int kPredWarps = 8;  // per tile
+constexpr int kPredThreads = (2 * kPredWarps + 2) * 32;
+constexpr int kPredK = 256;                          // features per piece
+constexpr int kPredBox = 128 * me::umma::kBK * 2;  // a box of weights
+constexpr int kPredStage = 2 * kPredBox;           // 64 inputs of a layer
+constexpr int kPredStages = 3;
+constexpr int kPredA = (kPredK / me::umma::kBK) * me::umma::kStageA;
+constexpr int kPredBars = 128;
+constexpr int kPredSmem = 2 * kPredA + kPredStages * kPredStage + kPredBars + 2 * 128 * 4;
+
+struct PredNet {
+  const float *bias[kLayers];
+  const float *fmean, *fistd, *tmean, *tstd;
+};
+
+// values k and k + 1 (k even, so both or neither are in) of a profile
+template <bool VEC>
+__device__ __forceinline__ double2 load_pair(const double *p, bool in) {
+  if (!in) return make_double2(0.0, 0.0);
+  if (VEC) return __ldg(reinterpret_cast<const double2 *>(p));
+  return make_double2(__ldg(p), __ldg(p + 1));
+}
+
+template <bool VEC>
+__global__ void __launch_bounds__(kPredThreads, 1)
+    mlp_predict_kernel(const __grid_constant__ CUtensorMap w0,
+                       const __grid_constant__ CUtensorMap w1,
+                       const __grid_constant__ CUtensorMap w2,
+                       const __grid_constant__ CUtensorMap w3, const PredNet net,
+                       const double *__restrict__ prof, long long n, int nl, int nip,
+                       double *__restrict__ par, int *__restrict__ err) {
+  using namespace me::umma;
+  extern __shared__ __align__(1024) uint8_t pred_smem[];
+  const uint32_t base = smem_u32(pred_smem);
+  const uint32_t sW = base + 2 * kPredA, bars = sW + kPredStages * kPredStage;
+  // full[s] = bars + 8 s, empty[s] after them, then done[tile]
+  const uint32_t done = bars + 8 * 2 * kPredStages;
+  uint32_t *misc = reinterpret_cast<uint32_t *>(pred_smem + (done + 16 - base));
+  volatile uint32_t *abort_flag = misc + 1;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp == 0) {
+    tmem_alloc(smem_u32(misc), 512);
+    tmem_relinquish();
+  }
+  if (threadIdx.x == 32) {
+    for (int s = 0; s < 2 * kPredStages + 2; s++) mbar_init(bars + 8 * s, 1);
+    *abort_flag = (base & 1023u) ? 1u : 0u;
+    if (base & 1023u) atomicExch(err, 1);  // the tiles need their alignment
+    mbar_fence_init();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = misc[0];
+  const long long tiles = (n + kBM - 1) / kBM;
+  const int pieces = (nip + kPredK - 1) / kPredK;
+  const int last_blocks = (nip - (pieces - 1) * kPredK + kBK - 1) / kBK;
+  // tile g of this CTA's k-th pair: blockIdx.x + (2 k + g) gridDim.x
+  const long long mine0 = (tiles - 1 - blockIdx.x) / gridDim.x + 1;  // (grid <= tiles)
+
+  // Stages of weights in the order the MMAs use them: per phase (a piece of the
+  // first layer, or a layer) and tile, its blocks of 64 inputs.
+  const int phases = pieces + 3;
+  auto blocks_of = [&](int ph) { return ph == pieces - 1 ? last_blocks : 4; };
+  if (warp == 2 * kPredWarps + 1) {
+    if (lane == 0 && !*abort_flag) {
+      uint32_t st = 0, par = 1;  // parity that empty[st] waits for (fresh: passes)
+      bool dead = false;
+      for (int todo = (int)mine0; todo > 0 && !dead; todo -= 2) {
+        if (VEC)  // the next pair's profiles into L2
+          for (int g = 2; g < 4 && g < todo; g++) {
+            const long long r = (blockIdx.x + (mine0 - todo + g) * gridDim.x) * kBM;
+            l2_prefetch(prof + (size_t)r * 4 * nl,
+                        (uint32_t)min((long long)kBM, n - r) * (uint32_t)nl * 32u);
+          }
+        for (int ph = 0; ph < phases && !dead; ph++)
+          for (int g = 0; g < 2 && g < todo && !dead; g++)
+            for (int kb = 0; kb < blocks_of(ph); kb++) {
+              if (!mbar_wait(bars + 8 * (kPredStages + st), par)) {
+                dead = true;  // (or the MMAs have stopped)
+                break;
+              }
+              const uint32_t full = bars + 8 * st, dst = sW + st * kPredStage;
+              if (ph == phases - 1) {
+                mbar_expect_tx(full, 32 * kBK * 2);
+                tma_load_2d(dst, &w3, full, kb * kBK, 0);
+              } else {
+                const CUtensorMap *w = ph < pieces ? &w0 : ph == pieces ? &w1 : &w2;
+                const int k = (ph < pieces ? ph * kPredK : 0) + kb * kBK;
+                mbar_expect_tx(full, kPredStage);
+                tma_load_2d(dst, w, full, k, 0);
+                tma_load_2d(dst + kPredBox, w, full, k, 128);
+              }
+              if (++st == kPredStages) st = 0, par ^= 1;
+            }
+      }
+      if (dead) {
+        *abort_flag = 1;
+        atomicExch(err, 2);
+        // copies that no MMA will read: let them land
+        for (uint32_t i = 0; i < kPredStages; i++)
+          mbar_wait(bars + 8 * i, i < st ? par ^ 1 : par);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 2 * kPredWarps) {
+    uint32_t st = 0, par = 0;
+    bool dead = *abort_flag != 0;
+    const uint64_t descW = sw128_kmajor_desc(sW);
+    for (int todo = (int)mine0; todo > 0; todo -= 2)
+      for (int ph = 0; ph < phases; ph++)
+        for (int g = 0; g < 2 && g < todo; g++) {
+          if (g == 0)
+            asm volatile("bar.sync 1, %0;" ::"n"((kPredWarps + 1) * 32) : "memory");
+          else
+            asm volatile("bar.sync 2, %0;" ::"n"((kPredWarps + 1) * 32) : "memory");
+          tc_fence_after();
+          if (lane == 0) {
+            const uint32_t idesc = idesc_bf16_f32(kBM, ph == phases - 1 ? 32 : 256);
+            uint64_t da = sw128_kmajor_desc(base + g * kPredA);
+            const uint32_t d = tmem + (uint32_t)(g * 256);
+            const int count = blocks_of(ph);
+            const bool fresh = ph == 0 || ph >= pieces;
+            for (int kb = 0; kb < count && !dead; kb++) {
+              if (!mbar_wait(bars + 8 * st, par)) {
+                dead = true;
+                atomicExch(err, 1);
+                break;
+              }
+              tc_fence_after();
+              // (a slice's address enters its descriptor in units of 16 bytes)
+              const uint64_t db = descW + (uint64_t)(st * (kPredStage >> 4));
+              umma_bf16(d, da, db, idesc, !(fresh && kb == 0));
+              umma_bf16(d, da + 2, db + 2, idesc, 1);
+              umma_bf16(d, da + 4, db + 4, idesc, 1);
+              umma_bf16(d, da + 6, db + 6, idesc, 1);
+              mma_commit(bars + 8 * (kPredStages + st));
+              da += kStageA >> 4;
+              if (++st == kPredStages) st = 0, par ^= 1;
+            }
+            if (dead) {
+              *abort_flag = 1;
+              mbar_arrive(done + 8 * g);
+            } else {
+              mma_commit(done + 8 * g);
+            }
+          }
+          __syncwarp();
+        }
+  } else {
+    const int g = warp / kPredWarps, gw = warp % kPredWarps;
+    uint8_t *tileA = pred_smem + g * kPredA;
+    float *s_imax = reinterpret_cast<float *>(pred_smem + (bars + kPredBars - base)) + g * 128;
+    uint32_t phase = 0;
+    auto publish = [&]() {  // the A tile is written and the accumulator read
+      fence_smem_to_async();
+      tc_fence_before();
+      if (g == 0)
+        asm volatile("bar.arrive 1, %0;" ::"n"((kPredWarps + 1) * 32) : "memory");
+      else
+        asm volatile("bar.arrive 2, %0;" ::"n"((kPredWarps + 1) * 32) : "memory");
+    };
+    auto group_sync = [&]() {
+      if (g == 0)
+        asm volatile("bar.sync 3, %0;" ::"n"(kPredWarps * 32) : "memory");
+      else
+        asm volatile("bar.sync 4, %0;" ::"n"(kPredWarps * 32) : "memory");
+    };
+    auto finished = [&]() {  // this phase's MMAs are done
+      if (!mbar_wait(done + 8 * g, phase & 1u)) {
+        *abort_flag = 1;
+        atomicExch(err, 3);
+      }
+      phase++;
+      tc_fence_after();
+    };
+    const int row = (gw & 3) * 32 + lane;  // this thread's row in the epilogues
+    const uint32_t trow = tmem + (uint32_t)(g * 256) + ((uint32_t)((gw & 3) * 32) << 16);
+    const int col0 = (gw >> 2) * 128;
+    const int nf = 4 * nl;
+    for (long long tile = blockIdx.x + (long long)g * gridDim.x; tile < tiles;
+         tile += 2LL * gridDim.x) {
+      const long long r0 = tile * kBM + gw * 16;  // this warp's rows of features
+      const double *p0 = prof + (size_t)r0 * nf;
+      // I_max, eight rows at a time: each lane's maxima, then a butterfly that
+      // halves the rows a lane holds at each of its first three steps; lanes
+      // 4 r .. 4 r + 3 end with row r's.
+      float my_inv[2];
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        double m[8];
+#pragma unroll
+        for (int r = 0; r < 8; r++) m[r] = 0.0;
+#pragma unroll 1
+        for (int k = 2 * lane; k < nl; k += 64) {
+          double2 v[8];
+#pragma unroll
+          for (int r = 0; r < 8; r++)
+            v[r] = load_pair<VEC>(p0 + (size_t)(8 * h + r) * nf + k, r0 + 8 * h + r < n);
+          const bool both = k + 1 < nl;
+#pragma unroll
+          for (int r = 0; r < 8; r++) m[r] = fmax(fmax(m[r], v[r].x), both ? v[r].y : 0.0);
+        }
+#pragma unroll
+        for (int w = 4; w; w >>= 1) {
+          const bool up = lane & (4 * w);
+#pragma unroll
+          for (int r = 0; r < w; r++) {
+            const double got = __shfl_xor_sync(0xffffffffu, up ? m[r] : m[r + w], 4 * w);
+            m[r] = fmax(up ? m[r + w] : m[r], got);
+          }
+        }
+        m[0] = fmax(m[0], __shfl_xor_sync(0xffffffffu, m[0], 2));
+        m[0] = fmax(m[0], __shfl_xor_sync(0xffffffffu, m[0], 1));
+        my_inv[h] = m[0] > 0 ? (float)(1.0 / m[0]) : 0.f;
+        if (!(lane & 3)) s_imax[gw * 16 + 8 * h + (lane >> 2)] = (float)m[0];
+      }
+      for (int pc = 0; pc < pieces; pc++) {
+        if (pc) finished();  // the piece before has been read
+        const int blocks = pc < pieces - 1 ? kPredK / kBK : last_blocks;
+#pragma unroll 1
+        for (int b = 0; b < blocks; b++) {
+          const int k = pc * kPredK + b * kBK + 2 * lane;
+          const bool in = k < nf;
+          double2 v[16];
+#pragma unroll
+          for (int r = 0; r < 16; r++)
+            v[r] = load_pair<VEC>(p0 + (size_t)r * nf + k, in && r0 + r < n);
+          float2 mean = make_float2(0.f, 0.f), istd = mean;
+          if (in) {
+            mean = __ldg(reinterpret_cast<const float2 *>(net.fmean + k));
+            istd = __ldg(reinterpret_cast<const float2 *>(net.fistd + k));
+          }
+#pragma unroll
+          for (int r = 0; r < 16; r++) {
+            const float inv = __shfl_sync(0xffffffffu, my_inv[r >> 3], 4 * (r & 7));
+            const float f0 =
+                (feature_value(k < nl ? 0 : 1, (float)v[r].x, inv) - mean.x) * istd.x;
+            const float f1 =
+                (feature_value(k + 1 < nl ? 0 : 1, (float)v[r].y, inv) - mean.y) * istd.y;
+            *reinterpret_cast<__nv_bfloat162 *>(
+                tileA + sw128_offset(gw * 16 + r, b * kBK + 2 * lane)) =
+                __floats2bfloat162_rn(in ? f0 : 0.f, in ? f1 : 0.f);  // (zeros in the padding)
+          }
+        }
+        publish();
+      }
+      for (int l = 0; l < 3; l++) {
+        finished();
+        const float *bias = net.bias[l];
+#pragma unroll 1
+        for (int c = col0; c < col0 + 128; c += 16) {
+          float bv[16], v[16];
+#pragma unroll
+          for (int j = 0; j < 16; j += 4) {
+            const float4 f = __ldg(reinterpret_cast<const float4 *>(bias + c + j));
+            bv[j] = f.x, bv[j + 1] = f.y, bv[j + 2] = f.z, bv[j + 3] = f.w;
+          }
+          tmem_ld16(trow + (uint32_t)c, v);
+#pragma unroll
+          for (int j = 0; j < 16; j++) v[j] += bv[j];
+          uint32_t pk[8];
+#pragma unroll
+          for (int j = 0; j < 8; j++) {
+            const __nv_bfloat162 h = __floats2bfloat162_rn(gelu_f(v[2 * j]), gelu_f(v[2 * j + 1]));
+            pk[j] = *reinterpret_cast<const uint32_t *>(&h);
+          }
+          *reinterpret_cast<uint4 *>(tileA + sw128_offset(row, c)) =
+              make_uint4(pk[0], pk[1], pk[2], pk[3]);
+          *reinterpret_cast<uint4 *>(tileA + sw128_offset(row, c + 8)) =
+              make_uint4(pk[4], pk[5], pk[6], pk[7]);
+        }
+        publish();
+      }
+      finished();
+      group_sync();  // s_imax is whole
+      if (gw < 4) {
+        float y[16];
+        tmem_ld16(trow, y);
+        const long long i = tile * kBM + row;
+#pragma unroll
+        for (int j = 0; j < kOut; j++) y[j] += __ldg(net.bias[3] + j);
+        if (i < n && !*abort_flag)
+          decode_row(y, net.tmean, net.tstd, s_imax[row], par + (size_t)i * 9);
+      }
+      group_sync();  // the next tile's I_max must not overtake the decode
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem, 512);
+}
+
+bool predict_kernel_ready() {
+  const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  return cudaFuncSetAttribute(mlp_predict_kernel<true>, a, kPredSmem) == cudaSuccess &&
+         cudaFuncSetAttribute(mlp_predict_kernel<false>, a, kPredSmem) == cudaSuccess;
 }
 
 // ---------------------------------------------------------------------------
@@ -1104,6 +1436,12 @@ namespace me {
 int plan_devplan(const me_plan *p, DevPlan *out, int *device);
 
 int mlp_gemm_status(me_mlp *m) { return gemm_status(m); }
+
+long long mlp_predict_launches(const me_mlp *m, long long npix) {
+  return m->gemm_path == GemmPath::tcgen05 && device_facts().pred_ok
+             ? 1
+             : kMlpPredLaunches * ((npix + kMlpPredChunk - 1) / kMlpPredChunk);
+}
 }  // namespace me
 
 extern "C" int me_mlp_train_params_default(me_mlp_train_params *tp) {
@@ -1253,6 +1591,37 @@ extern "C" int me_mlp_train(me_plan *plan, const me_mlp_train_params *tp, me_mlp
   return ME_OK;
 }
 
+// The inference in one kernel, where the tcgen05 kernels are chosen and can run;
+// false: nothing was launched.
+static bool predict_fused(me_mlp *m, const double *d_prof, long npix, double *d_par,
+                          cudaStream_t st) {
+  const DeviceFacts &dv = device_facts();
+  if (m->gemm_path != GemmPath::tcgen05 || !m->gerr.p || !dv.pred_ok || dv.sms <= 0) return false;
+  CUtensorMap w[kLayers];
+  for (int l = 0; l < kLayers; l++)
+    if (!cached_tile_map(&m->maps, &w[l], m->wb[l].as<bf16>(), m->dout[l], m->din[l],
+                         l < kLayers - 1 ? 128 : kOutPad))
+      return false;
+  PredNet net;
+  for (int l = 0; l < kLayers; l++) net.bias[l] = m->b[l].as<float>();
+  net.fmean = m->fmean.as<float>();
+  net.fistd = m->fistd.as<float>();
+  net.tmean = m->tmean.as<float>();
+  net.tstd = m->tstd.as<float>();
+  const long long tiles = ((long long)npix + me::umma::kBM - 1) / me::umma::kBM;
+  const unsigned grid = (unsigned)(tiles < dv.sms ? tiles : dv.sms);
+  auto go = [&](auto kernel) {
+    kernel<<<grid, kPredThreads, kPredSmem, st>>>(w[0], w[1], w[2], w[3], net, d_prof, npix, m->nl,
+                                                  m->nip, d_par, m->gerr.as<int>());
+  };
+  if ((reinterpret_cast<uintptr_t>(d_prof) & 15) == 0)
+    go(mlp_predict_kernel<true>);
+  else
+    go(mlp_predict_kernel<false>);
+  m->gemm_launches[(int)GemmPath::tcgen05]++;
+  return true;
+}
+
 extern "C" int me_mlp_predict_device(me_mlp *m, const double *d_prof, long npix, double *d_par,
                                      void *stream) {
   if (!m || (npix > 0 && (!d_prof || !d_par)) || npix < 0)
@@ -1260,6 +1629,14 @@ extern "C" int me_mlp_predict_device(me_mlp *m, const double *d_prof, long npix,
   if (npix == 0) return ME_OK;
   MCK(cudaSetDevice(m->device));
   cudaStream_t st = (cudaStream_t)stream;
+  if (predict_fused(m, d_prof, npix, d_par, st)) {
+    MCK(cudaGetLastError());
+    if (!stream) {
+      MCK(cudaStreamSynchronize(st));
+      return gemm_status(m);
+    }
+    return ME_OK;
+  }
   const int chunk = (int)(npix < me::kMlpPredChunk ? (npix + 255) / 256 * 256 : me::kMlpPredChunk);
   int rc = ensure_batch(m, chunk);
   if (rc) return rc;

@@ -84,11 +84,15 @@ __device__ __forceinline__ unsigned long long now_ns() {
 // Waits for the completion of the phase of parity `parity`; false when it has
 // not completed within kWaitNs (the caller records an error and stops).
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-  if (mbar_try(bar, parity)) return true;
-  const unsigned long long t0 = now_ns();
+  // (the timer is read only once the first tries have failed)
+  unsigned long long t0 = 0;
   for (uint32_t it = 1; it < (1u << 26); it++) {
     if (mbar_try(bar, parity)) return true;
-    if ((it & 63) == 0 && now_ns() - t0 > kWaitNs) return false;
+    if ((it & 63) == 0) {
+      const unsigned long long t = now_ns();
+      if (!t0) t0 = t;
+      if (t - t0 > kWaitNs) return false;
+    }
   }
   return false;
 }
@@ -103,6 +107,11 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
       " [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
       "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y)
       : "memory");
+}
+
+// `bytes` from p on into L2; both multiples of 16
+__device__ __forceinline__ void l2_prefetch(const void *p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
 // Tensor memory: allocate / free `ncols` columns (a power of two >= 32) for
@@ -161,6 +170,24 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                    bar)
                : "memory");
+}
+
+// one plain arrival on `bar`
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+// makes this thread's shared-memory writes visible to the tensor cores
+__device__ __forceinline__ void fence_smem_to_async() {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
+// Byte offset of element (row, k) in a stack of K-major, 128-byte-swizzled
+// tiles of kBM rows x kBK values, as TMA writes them: 16-byte pieces of a row's
+// 128 bytes are permuted by the row's number modulo 8.
+__device__ __forceinline__ uint32_t sw128_offset(int row, int k) {
+  return (uint32_t)(k / kBK) * kStageA + (uint32_t)row * 128 +
+         ((((uint32_t)(k % kBK) >> 3) ^ ((uint32_t)row & 7)) << 4) + ((uint32_t)k & 7) * 2;
 }
 
 // 16 consecutive FP32 columns of the warp's 32 tensor-memory lanes (lane i of
