@@ -553,7 +553,8 @@ int me_mlp_loss_grad(me_mlp *mlp, const float *x, const float *t, int rows, doub
 #define ME_GEMM_TCGEN05 0
 #define ME_GEMM_MMA_SYNC 1
 int me_mlp_set_gemm(me_mlp *mlp, int path);
-/* GEMM launches of each kernel since the initialiser was made. */
+/* GEMMs that each kind of kernel has run since the initialiser was made (a
+ * launch of the fused inference or training kernels runs several). */
 int me_mlp_gemm_launches(const me_mlp *mlp, long long *tcgen05, long long *mma_sync);
 
 /* One GEMM of the initialiser's kernels, for testing them: with A [m][r] and

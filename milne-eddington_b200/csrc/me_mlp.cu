@@ -34,6 +34,7 @@ namespace mlp {
 constexpr int kHidden = 256;
 constexpr int kOut = 10;
 constexpr int kLayers = 4;
+constexpr int kOutRows = 32;  // rows of the last layer's weights (10 used, zeros past)
 typedef __nv_bfloat16 bf16;
 
 // ---------------------------------------------------------------------------
@@ -163,11 +164,11 @@ __global__ void __launch_bounds__(128) gemm_kernel(const bf16 *__restrict__ A,
 // release, 3: accumulator), drains what it issued, frees its tensor memory
 // and leaves C unwritten.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128, 1)
-    umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA,
-                     const __grid_constant__ CUtensorMap tmB, int M, int N, int R, int bn,
-                     const float *__restrict__ bias, float *__restrict__ Z, int gelu,
-                     bf16 *__restrict__ Y, float *__restrict__ Yf, int *__restrict__ err) {
+__device__ __forceinline__ void umma_tile(const CUtensorMap *tmA, const CUtensorMap *tmB, int m0,
+                                          int n0, int bn, int kbeg, int rz, bool split, int M,
+                                          int N, const float *__restrict__ bias,
+                                          float *__restrict__ Z, int gelu, bf16 *__restrict__ Y,
+                                          float *__restrict__ Yf, int *__restrict__ err) {
   using namespace me::umma;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -200,8 +201,6 @@ __global__ void __launch_bounds__(128, 1)
   tc_fence_after();
   const uint32_t tmem = misc[0];
 
-  const int m0 = blockIdx.y * kBM, n0 = blockIdx.x * bn;
-  const int rz = R / (int)gridDim.z, kbeg = blockIdx.z * rz;
   const int nk = (rz + kBK - 1) / kBK;
   const uint32_t tx = (uint32_t)(kBM + bn) * kBK * 2;
 
@@ -212,8 +211,8 @@ __global__ void __launch_bounds__(128, 1)
       for (; loaded < nk && loaded < kStages; loaded++) {
         const uint32_t full = bars + 8 * loaded;
         mbar_expect_tx(full, tx);
-        tma_load_2d(sA + loaded * kStageA, &tmA, full, kbeg + loaded * kBK, m0);
-        tma_load_2d(sB + loaded * stB, &tmB, full, kbeg + loaded * kBK, n0);
+        tma_load_2d(sA + loaded * kStageA, tmA, full, kbeg + loaded * kBK, m0);
+        tma_load_2d(sB + loaded * stB, tmB, full, kbeg + loaded * kBK, n0);
       }
       for (; kb < nk; kb++) {
         const int s = kb % kStages;
@@ -236,8 +235,8 @@ __global__ void __launch_bounds__(128, 1)
           }
           const uint32_t full = bars + 8 * ls;
           mbar_expect_tx(full, tx);
-          tma_load_2d(sA + ls * kStageA, &tmA, full, kbeg + loaded * kBK, m0);
-          tma_load_2d(sB + ls * stB, &tmB, full, kbeg + loaded * kBK, n0);
+          tma_load_2d(sA + ls * kStageA, tmA, full, kbeg + loaded * kBK, m0);
+          tma_load_2d(sB + ls * stB, tmB, full, kbeg + loaded * kBK, n0);
           loaded++;
         }
       }
@@ -267,9 +266,11 @@ __global__ void __launch_bounds__(128, 1)
       tmem_ld16(trow + (uint32_t)c, v);
       if (row >= M) continue;
       const size_t o = (size_t)row * N + n;
-      if (gridDim.z > 1) {
+      if (split) {
 #pragma unroll
-        for (int j = 0; j < 16; j++) atomicAdd(Yf + o + j, v[j]);
+        for (int j = 0; j < 16; j += 4)
+          atomicAdd(reinterpret_cast<float4 *>(Yf + o + j),
+                    make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]));
         continue;
       }
       if (bias) {
@@ -306,6 +307,16 @@ __global__ void __launch_bounds__(128, 1)
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, ncols);
+}
+
+__global__ void __launch_bounds__(128, 1)
+    umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA,
+                     const __grid_constant__ CUtensorMap tmB, int M, int N, int R, int bn,
+                     const float *__restrict__ bias, float *__restrict__ Z, int gelu,
+                     bf16 *__restrict__ Y, float *__restrict__ Yf, int *__restrict__ err) {
+  const int rz = R / (int)gridDim.z;
+  umma_tile(&tmA, &tmB, blockIdx.y * me::umma::kBM, blockIdx.x * bn, bn, blockIdx.z * rz, rz,
+            gridDim.z > 1, M, N, bias, Z, gelu, Y, Yf, err);
 }
 
 // cuTensorMapEncodeTiled from the driver, looked up once through the runtime
@@ -384,10 +395,11 @@ bool cached_tile_map(TileMapCache *c, CUtensorMap *map, const bf16 *p, int rows,
 // and whether the kernel's shared-memory limit has been raised.
 struct DeviceFacts {
   int sms = 0;
-  bool smem_ok = false, pred_ok = false;
+  bool smem_ok = false, pred_ok = false, step_ok = false;
 };
 
-bool predict_kernel_ready();  // (below, with the kernel)
+bool predict_kernel_ready();  // (below, with the kernels)
+bool step_kernels_ready();
 
 const DeviceFacts &device_facts() {
   static DeviceFacts facts[64];
@@ -404,6 +416,7 @@ const DeviceFacts &device_facts() {
     f.smem_ok = cudaFuncSetAttribute(umma_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      me::umma::kSmemMax) == cudaSuccess;
     f.pred_ok = predict_kernel_ready();
+    f.step_ok = f.smem_ok && step_kernels_ready();
     facts[dev] = f;
   });
   return facts[dev];
@@ -992,6 +1005,333 @@ bool predict_kernel_ready() {
 }
 
 // ---------------------------------------------------------------------------
+// A training step up to the gradients' operands in one kernel: the batch's
+// gather, the forward pass, the loss and the backward pass to every layer's
+// dZ.  A CTA takes 32 rows of the batch, so that a batch of 4096 fills 128 SMs,
+// and computes each layer transposed: the weights are the 256 (two times 128)
+// rows of the MMA and the batch rows its columns.  So a thread's accumulators
+// are 16 batch rows of one neuron: the layer's output leaves for the weight
+// gradient's transposed operand as 32-byte stores, the bias is one value, the
+// bias gradient a sum in registers, and the pre-activations of the three hidden
+// layers stay in registers until the backward pass asks for them.  The next
+// operand is written to shared memory as in mlp_predict_kernel, whose warps of
+// loads and of MMAs this has too; a layer's weights fill the four stages, so
+// they arrive during the epilogue before them.  The values are those of
+// gather_kernel, the GEMMs and their epilogues, mse_grad_kernel and
+// gelu_back_kernel (which the mma.sync path runs), each rounded to BF16 at the
+// same places.  A CTA's 32 us at a batch of 4096: gathering 2, the epilogues'
+// instructions 12 (erff, and in the backward pass expf), the MMAs and the
+// weights they wait for 11.  With mlp_wgrad_kernel (12 us) and adam_kernel (7)
+// a step takes 55 us, as 44 launches it took 248; with a batch of 256, 48 (190);
+// of 65,536, 520 (1,250).
+// ---------------------------------------------------------------------------
+constexpr int kStepRows = 32, kStepWarps = 16;
+constexpr int kStepThreads = (kStepWarps + 2) * 32;
+constexpr int kStepStages = 4;
+constexpr int kStepBlock = kStepRows * me::umma::kBK * 2;  // 64 inputs of the batch rows
+constexpr int kStepBars = 128;
+constexpr int kStepSmem = kStepStages * kPredStage + 4 * kStepBlock + kStepBars;
+
+struct StepMaps {
+  CUtensorMap w[kLayers];  // W [dout][din]
+  CUtensorMap t[kLayers];  // W^T [din][dout], layers 1..
+};
+struct StepNet {
+  const float *bias[kLayers];
+  bf16 *xt;               // [nip][B]: the batch, transposed
+  bf16 *at[kLayers - 1];  // [256][B]: the hidden layers' outputs
+  bf16 *dzt[kLayers];     // [dout][B]: dZ
+  float *gb[kLayers];     // += the bias gradients
+};
+
+__device__ __forceinline__ uint32_t step_offset(int row, int k) {
+  return (uint32_t)(k / me::umma::kBK) * kStepBlock + (uint32_t)row * 128 +
+         ((((uint32_t)(k % me::umma::kBK) >> 3) ^ ((uint32_t)row & 7)) << 4) +
+         ((uint32_t)k & 7) * 2;
+}
+
+__global__ void __launch_bounds__(kStepThreads, 1)
+    mlp_step_kernel(const __grid_constant__ StepMaps maps, const __grid_constant__ StepNet net,
+                    const bf16 *__restrict__ X, const long long *__restrict__ idx,
+                    const float *__restrict__ T, int B, int nip, double *__restrict__ loss,
+                    int *__restrict__ err) {
+  using namespace me::umma;
+  extern __shared__ __align__(1024) uint8_t step_smem[];
+  const uint32_t base = smem_u32(step_smem);
+  uint8_t *tile = step_smem + kStepStages * kPredStage;
+  const uint32_t sX = base + kStepStages * kPredStage, bars = sX + 4 * kStepBlock;
+  // full[s] = bars + 8 s, empty[s] after them, then done
+  const uint32_t done = bars + 8 * 2 * kStepStages;
+  uint32_t *misc = reinterpret_cast<uint32_t *>(step_smem + (done + 8 - base));
+  volatile uint32_t *abort_flag = misc + 1;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp == 0) {
+    tmem_alloc(smem_u32(misc), 64);
+    tmem_relinquish();
+  }
+  if (threadIdx.x == 32) {
+    for (int s = 0; s < 2 * kStepStages + 1; s++) mbar_init(bars + 8 * s, 1);
+    *abort_flag = (base & 1023u) ? 1u : 0u;
+    if (base & 1023u) atomicExch(err, 1);  // the tiles need their alignment
+    mbar_fence_init();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = misc[0];
+  const int row0 = blockIdx.x * kStepRows;
+  const int pieces = (nip + kPredK - 1) / kPredK;
+  const int last_blocks = (nip - (pieces - 1) * kPredK + kBK - 1) / kBK;
+  // phases: the first layer's pieces, layers 1 and 2, the outputs, then back
+  // through the outputs' weights and layers 2 and 1
+  const int phases = pieces + 6, out = pieces + 2;
+  auto blocks_of = [&](int ph) { return ph == pieces - 1 ? last_blocks : ph == out + 1 ? 1 : 4; };
+
+  if (warp == kStepWarps + 1) {
+    if (lane == 0 && !*abort_flag) {
+      uint32_t st = 0, par = 1;  // parity that empty[st] waits for (fresh: passes)
+      bool dead = false;
+      for (int ph = 0; ph < phases && !dead; ph++) {
+        const CUtensorMap *w = ph < pieces ? &maps.w[0]
+                               : ph <= out ? &maps.w[ph - pieces + 1]
+                                           : &maps.t[kLayers - (ph - out)];
+        for (int kb = 0; kb < blocks_of(ph); kb++) {
+          if (!mbar_wait(bars + 8 * (kStepStages + st), par)) {
+            dead = true;  // (or the MMAs have stopped)
+            break;
+          }
+          const uint32_t full = bars + 8 * st, dst = base + st * kPredStage;
+          const int k = (ph < pieces ? ph * kPredK : 0) + kb * kBK;
+          mbar_expect_tx(full, ph == out ? 32 * kBK * 2 : kPredStage);
+          tma_load_2d(dst, w, full, k, 0);
+          if (ph != out) tma_load_2d(dst + kPredBox, w, full, k, 128);
+          if (++st == kStepStages) st = 0, par ^= 1;
+        }
+      }
+      if (dead) {
+        *abort_flag = 1;
+        atomicExch(err, 2);
+        // copies that no MMA will read: let them land
+        for (uint32_t i = 0; i < kStepStages; i++)
+          mbar_wait(bars + 8 * i, i < st ? par ^ 1 : par);
+      }
+    }
+    __syncwarp();
+  } else if (warp == kStepWarps) {
+    uint32_t st = 0, par = 0;
+    bool dead = *abort_flag != 0;
+    const uint64_t descW = sw128_kmajor_desc(base);
+    const uint32_t idesc = idesc_bf16_f32(kBM, kStepRows);
+    for (int ph = 0; ph < phases; ph++) {
+      asm volatile("bar.sync 1, %0;" ::"n"((kStepWarps + 1) * 32) : "memory");
+      tc_fence_after();
+      if (lane == 0) {
+        uint64_t db = sw128_kmajor_desc(sX);
+        const int count = blocks_of(ph);
+        const bool fresh = ph == 0 || ph >= pieces;
+        for (int kb = 0; kb < count && !dead; kb++) {
+          if (!mbar_wait(bars + 8 * st, par)) {
+            dead = true;
+            atomicExch(err, 1);
+            break;
+          }
+          tc_fence_after();
+          // (a slice's address enters its descriptor in units of 16 bytes)
+          const uint64_t da = descW + (uint64_t)(st * (kPredStage >> 4));
+          const int slices = ph == out + 1 ? kOutRows / 16 : 4;
+          for (int k = 0; k < slices; k++) {  // (the halves in turn: each MMA waits for its
+            const uint32_t add = !(fresh && kb == 0 && k == 0);  // accumulator's last)
+            umma_bf16(tmem, da + 2 * k, db + 2 * k, idesc, add);
+            if (ph != out)
+              umma_bf16(tmem + kStepRows, da + (kPredBox >> 4) + 2 * k, db + 2 * k, idesc, add);
+          }
+          mma_commit(bars + 8 * (kStepStages + st));
+          db += kStepBlock >> 4;
+          if (++st == kStepStages) st = 0, par ^= 1;
+        }
+        if (dead) {
+          *abort_flag = 1;
+          mbar_arrive(done);
+        } else {
+          mma_commit(done);
+        }
+      }
+      __syncwarp();
+    }
+  } else {
+    uint32_t phase = 0;
+    auto publish = [&]() {  // the operand is written and the accumulator read
+      fence_smem_to_async();
+      tc_fence_before();
+      asm volatile("bar.arrive 1, %0;" ::"n"((kStepWarps + 1) * 32) : "memory");
+    };
+    auto workers = [&]() {
+      asm volatile("bar.sync 2, %0;" ::"n"(kStepWarps * 32) : "memory");
+    };
+    auto finished = [&]() {  // this phase's MMAs are done
+      if (!mbar_wait(done, phase & 1u)) {
+        *abort_flag = 1;
+        atomicExch(err, 3);
+      }
+      phase++;
+      tc_fence_after();
+    };
+    // the batch
+    for (int pc = 0; pc < pieces; pc++) {
+      if (pc) finished();  // the piece before has been read
+      const int blocks = pc < pieces - 1 ? 4 : last_blocks;
+      for (int i = threadIdx.x; i < kStepRows * blocks * 8; i += kStepWarps * 32) {
+        const int r = i / (blocks * 8), c = i % (blocks * 8), k = pc * kPredK + c * 8;
+        uint4 v = make_uint4(0, 0, 0, 0);  // zeros past the features
+        if (k < nip)
+          v = __ldg(reinterpret_cast<const uint4 *>(X + (size_t)__ldg(idx + row0 + r) * nip + k));
+        *reinterpret_cast<uint4 *>(tile + step_offset(r, c * 8)) = v;
+      }
+      publish();
+      workers();
+      for (int i = threadIdx.x; i < 2 * blocks * kBK; i += kStepWarps * 32) {
+        const int c = i >> 1, r = (i & 1) * 16, k = pc * kPredK + c;
+        if (k >= nip) continue;
+        uint32_t pk[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+          pk[j] = *reinterpret_cast<const uint16_t *>(tile + step_offset(r + 2 * j, c)) |
+                  (uint32_t)*reinterpret_cast<const uint16_t *>(
+                      tile + step_offset(r + 2 * j + 1, c))
+                      << 16;
+        uint4 *o = reinterpret_cast<uint4 *>(net.xt + (size_t)k * B + row0 + r);
+        o[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+        o[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+      }
+      workers();  // the tile has been read
+    }
+    // this thread's neuron and 16 batch rows
+    const int neuron = ((warp >> 2) & 1) * 128 + (warp & 3) * 32 + lane, r16 = (warp >> 3) * 16;
+    const uint32_t acc = tmem + (uint32_t)(((warp >> 2) & 1) * kStepRows + r16) +
+                         ((uint32_t)((warp & 3) * 32) << 16);
+    // BF16 values as the next operand, and then as the weight gradient's (a fence
+    // for the first would wait for the second's stores)
+    auto put_next = [&](const float v[16], int n) {
+#pragma unroll
+      for (int j = 0; j < 16; j++)
+        *reinterpret_cast<bf16 *>(tile + step_offset(r16 + j, n)) = __float2bfloat16(v[j]);
+    };
+    auto put_grad = [&](const float v[16], bf16 *outT, int n) {
+      uint32_t pk[8];
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+        pk[j] = *reinterpret_cast<const uint32_t *>(&h);
+      }
+      uint4 *o = reinterpret_cast<uint4 *>(outT + (size_t)n * B + row0 + r16);
+      o[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+      o[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+    };
+    auto column_sum = [&](const float v[16]) {  // of the rounded values
+      float t = 0.f;
+#pragma unroll
+      for (int j = 0; j < 16; j++) t += __bfloat162float(__float2bfloat16(v[j]));
+      return t;
+    };
+    float z[kLayers - 1][16];
+#pragma unroll
+    for (int l = 0; l < kLayers - 1; l++) {
+      const float b = __ldg(net.bias[l] + neuron);
+      finished();
+      tmem_ld16(acc, z[l]);
+      float h[16];
+#pragma unroll
+      for (int j = 0; j < 16; j++) {
+        z[l][j] += b;
+        h[j] = gelu_f(z[l][j]);
+      }
+      put_next(h, neuron);
+      publish();
+      put_grad(h, net.at[l], neuron);
+    }
+    if ((warp & 7) == 0) {  // the outputs: lane's, 16 rows
+      float v[16], t[16], sq = 0.f;
+      const float b = __ldg(net.bias[kLayers - 1] + lane);
+#pragma unroll
+      for (int j = 0; j < 16; j++)
+        t[j] = lane < kOut ? __ldg(T + (size_t)__ldg(idx + row0 + r16 + j) * kOut + lane) : 0.f;
+      finished();
+      tmem_ld16(acc, v);
+#pragma unroll
+      for (int j = 0; j < 16; j++) {
+        float g = 0.f;
+        if (lane < kOut) {
+          const float d = v[j] + b - t[j];
+          g = 2.f * d / (float)(B * kOut);
+          sq += d * d;
+        }
+        v[j] = g;
+      }
+      put_next(v, lane);
+      publish();
+      put_grad(v, net.dzt[kLayers - 1], lane);
+      atomicAdd(net.gb[kLayers - 1] + lane, column_sum(v));
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+      if (lane == 0) atomicAdd(loss, (double)sq / (double)(B * kOut));
+    } else {
+      finished();
+      publish();
+    }
+#pragma unroll
+    for (int l = kLayers - 2; l >= 0; l--) {
+      float v[16];
+      finished();
+      tmem_ld16(acc, v);
+#pragma unroll
+      for (int j = 0; j < 16; j++) v[j] *= gelu_grad(z[l][j]);
+      if (l > 0) {
+        put_next(v, neuron);
+        publish();
+      }
+      put_grad(v, net.dzt[l], neuron);
+      atomicAdd(net.gb[l] + neuron, column_sum(v));
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem, 64);
+}
+
+// The weight gradients of all layers in one launch, dW_l [dout][din] += dZ_l^T
+// [dout][B] times A_l^T [din][B], each a GEMM over the batch divided in `split`
+// shares whose CTAs add into dW.  blockIdx.y: the share; blockIdx.x: the 128 x
+// kGradN tiles of layer 0, then of the next layers.
+constexpr int kGradN = 128;
+struct GradMaps {
+  CUtensorMap a[kLayers], b[kLayers];
+};
+struct GradNet {
+  float *gw[kLayers];
+  int m[kLayers], n[kLayers], tiles[kLayers];
+};
+
+__global__ void __launch_bounds__(128, 1)
+    mlp_wgrad_kernel(const __grid_constant__ GradMaps maps,
+                     const __grid_constant__ GradNet net, int B,
+                     int *__restrict__ err) {
+  int l = 0, t = blockIdx.x;
+  while (l < kLayers - 1 && t >= net.tiles[l]) t -= net.tiles[l++];
+  const int across = (net.n[l] + kGradN - 1) / kGradN;
+  const int rz = B / (int)gridDim.y;
+  umma_tile(&maps.a[l], &maps.b[l], t / across * me::umma::kBM, t % across * kGradN, kGradN,
+            blockIdx.y * rz, rz, true, net.m[l], net.n[l], nullptr, nullptr, 0, nullptr,
+            net.gw[l], err);
+}
+
+bool step_kernels_ready() {
+  return cudaFuncSetAttribute(mlp_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              kStepSmem) == cudaSuccess &&
+         cudaFuncSetAttribute(mlp_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              me::umma::kSmemMax) == cudaSuccess;
+}
+
+// ---------------------------------------------------------------------------
 // loss and optimiser
 // ---------------------------------------------------------------------------
 // dY = 2 (Y - T) / (rows * kOut) for the batch rows idx[0..rows) (T standardised,
@@ -1051,25 +1391,37 @@ __global__ void bias_grad_kernel(const bf16 *dZ, int rows, int cols, int rows_pe
   }
 }
 
-// Adam (Kingma & Ba 2015) on FP32 master weights, refreshing the BF16 copy
-// and its transpose.  w is [rows][cols].
-__global__ void adam_kernel(float *w, float *m, float *v, const float *g, long long n, int cols,
-                            float lr, float b1, float b2, float eps, float c1, float c2,
-                            bf16 *wb, bf16 *wbt, int rows) {
+// Adam (Kingma & Ba 2015) on all FP32 master parameters at once, refreshing the BF16
+// weights and their transposes, and clearing the gradients for the next step.
+// Parameters, moments and gradients have one layout of n floats; layer l's
+// weights [rows][cols] start at off[l], its biases lie before off[l + 1].
+struct AdamNet {
+  float *w, *m, *v, *g;
+  long long n, off[kLayers];
+  int rows[kLayers], cols[kLayers];
+  bf16 *wb[kLayers], *wbt[kLayers];
+};
+
+__global__ void adam_kernel(const __grid_constant__ AdamNet net, float lr, float b1, float b2, float eps, float c1,
+                            float c2) {
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float gi = g[i];
-  const float mi = b1 * m[i] + (1.f - b1) * gi;
-  const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  const float wi = w[i] - lr * (mi * c1) / (sqrtf(vi * c2) + eps);
-  w[i] = wi;
-  if (wb) {
-    wb[i] = __float2bfloat16(wi);
-    const long long r = i / cols, c = i % cols;
-    wbt[(size_t)c * rows + r] = __float2bfloat16(wi);
-  }
+  if (i >= net.n) return;
+  const float gi = net.g[i];
+  net.g[i] = 0.f;
+  const float mi = b1 * net.m[i] + (1.f - b1) * gi;
+  const float vi = b2 * net.v[i] + (1.f - b2) * gi * gi;
+  net.m[i] = mi;
+  net.v[i] = vi;
+  const float wi = net.w[i] - lr * (mi * c1) / (sqrtf(vi * c2) + eps);
+  net.w[i] = wi;
+  int l = 0;
+#pragma unroll
+  for (int k = 1; k < kLayers; k++) l = i >= net.off[k] ? k : l;
+  const int j = (int)(i - net.off[l]), cols = net.cols[l], rows = net.rows[l];
+  if (j >= rows * cols) return;
+  const bf16 h = __float2bfloat16(wi);
+  net.wb[l][j] = h;
+  net.wbt[l][(size_t)(j % cols) * rows + j / cols] = h;
 }
 
 // gather rows idx[] of X [n][cols] into Xb [rows][cols]
@@ -1118,11 +1470,12 @@ namespace {
 
 using namespace me::mlp;
 
-constexpr int kOutPad = 32;      // output rows of the last layer (10 used, zero weights past)
+constexpr int kOutPad = kOutRows;
 
 struct DBuf {
   void *p = nullptr;
   size_t n = 0;
+  bool own = true;
   DBuf() = default;
   DBuf(const DBuf &) = delete;
   DBuf &operator=(const DBuf &) = delete;
@@ -1137,10 +1490,17 @@ struct DBuf {
       p = nullptr;
     return e;
   }
+  void view(void *q, size_t bytes) {  // a part of another buffer, which outlives this one
+    release();
+    p = q;
+    n = bytes;
+    own = false;
+  }
   void release() {
-    if (p) cudaFree(p);
+    if (p && own) cudaFree(p);
     p = nullptr;
     n = 0;
+    own = true;
   }
   template <class T>
   T *as() const {
@@ -1157,6 +1517,24 @@ int fail(int code, const std::string &m) { return me::record_error(code, m.c_str
       return fail(ME_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
+// Parts of one allocation, each on 256 bytes: ask for them, take the memory,
+// and the buffers are views of it.
+struct Arena {
+  struct Part {
+    DBuf *d;
+    size_t off, bytes;
+  };
+  std::vector<Part> parts;
+  size_t total = 0;
+  void add(DBuf &d, size_t bytes) {
+    parts.push_back({&d, total, bytes});
+    total += (bytes + 255) / 256 * 256;
+  }
+  void place(void *p) const {
+    for (const Part &q : parts) q.d->view(static_cast<char *>(p) + q.off, q.bytes);
+  }
+};
+
 inline unsigned nblk(long long n, int b = 256) { return (unsigned)((n + b - 1) / b); }
 
 }  // namespace
@@ -1168,13 +1546,18 @@ struct me_mlp {
   // per layer: FP32 master W [dout][din] and b, BF16 W and W^T, Adam moments, gradients
   DBuf w[kLayers], b[kLayers], wb[kLayers], wbt[kLayers], mw[kLayers], vw[kLayers], mb[kLayers],
       vb[kLayers], gw[kLayers], gb[kLayers];
-  DBuf fmean, fistd, tmean, tstd;  // feature and target standardisation (device)
+  DBuf fmean, fistd, tmean, tstd, tistd;  // feature and target standardisation (device)
   std::vector<float> h_fmean, h_fistd, h_tmean, h_tstd;
   long long adam_t = 0;
   // batch work buffers
-  int cap = 0;
-  DBuf xb, xbt, z[kLayers], a[kLayers], at[kLayers], yf, dyb, dybt, dh, dz, dzt, loss;
-  DBuf imax;
+  int cap = 0, step_cap = 0;
+  DBuf xb, xbt, z[kLayers], a[kLayers], at[kLayers], yf, dyb, dybt, dh, dz, dzt;
+  DBuf sxt, sat[kLayers - 1], sdzt[kLayers];  // operands of the weight gradients (mlp_step_kernel)
+  DBuf loss, imax;
+  // the allocations that the buffers above are parts of; the parameters, their
+  // moments and their gradients have one layout, of `flat` floats each
+  DBuf model, batch, step;
+  long long flat = 0;
   // GEMM kernel choice and the tcgen05 kernel's error flag (device int)
   GemmPath gemm_path = GemmPath::tcgen05;
   DBuf gerr;
@@ -1216,22 +1599,45 @@ long long param_count(const me_mlp *m) {
 int ensure_batch(me_mlp *m, int B) {
   if (B <= m->cap) return ME_OK;
   const size_t r = (size_t)B;
-  MCK(m->xb.ensure(r * m->nip * 2));
-  MCK(m->xbt.ensure(r * m->nip * 2));
+  Arena a;
+  a.add(m->xb, r * m->nip * 2);
+  a.add(m->xbt, r * m->nip * 2);
   for (int l = 0; l < kLayers; l++) {
-    MCK(m->z[l].ensure(r * m->dout[l] * 4));
-    MCK(m->a[l].ensure(r * m->dout[l] * 2));
-    MCK(m->at[l].ensure(r * m->dout[l] * 2));
+    a.add(m->z[l], r * m->dout[l] * 4);
+    a.add(m->a[l], r * m->dout[l] * 2);
+    a.add(m->at[l], r * m->dout[l] * 2);
   }
-  MCK(m->yf.ensure(r * kOutPad * 4));
-  MCK(m->dyb.ensure(r * kOutPad * 2));
-  MCK(m->dybt.ensure(r * kOutPad * 2));
-  MCK(m->dh.ensure(r * kHidden * 4));
-  MCK(m->dz.ensure(r * kHidden * 2));
-  MCK(m->dzt.ensure(r * kHidden * 2));
-  MCK(m->loss.ensure(sizeof(double)));
-  MCK(m->imax.ensure(r * 4));
+  a.add(m->yf, r * kOutPad * 4);
+  a.add(m->dyb, r * kOutPad * 2);
+  a.add(m->dybt, r * kOutPad * 2);
+  a.add(m->dh, r * kHidden * 4);
+  a.add(m->dz, r * kHidden * 2);
+  a.add(m->dzt, r * kHidden * 2);
+  a.add(m->imax, r * 4);
+  m->cap = 0;
+  MCK(m->batch.ensure(a.total));
+  a.place(m->batch.p);
   m->cap = B;
+  return ME_OK;
+}
+
+// the operands of the weight gradients of B rows, in `mem` where they fit
+int ensure_step(me_mlp *m, int B, void *mem, size_t bytes) {
+  if (!mem && B <= m->step_cap) return ME_OK;
+  Arena a;
+  a.add(m->sxt, (size_t)B * m->nip * 2);
+  for (int l = 0; l < kLayers; l++) {
+    if (l < kLayers - 1) a.add(m->sat[l], (size_t)B * m->dout[l] * 2);
+    a.add(m->sdzt[l], (size_t)B * m->dout[l] * 2);
+  }
+  if (a.total <= bytes) {
+    a.place(mem);
+    return ME_OK;
+  }
+  m->step_cap = 0;
+  MCK(m->step.ensure(a.total));
+  a.place(m->step.p);
+  m->step_cap = B;
   return ME_OK;
 }
 
@@ -1284,27 +1690,35 @@ int alloc_model(me_mlp *m, int nl) {
   m->nl = nl;
   m->nin = 4 * nl;
   m->nip = (m->nin + 31) / 32 * 32;
-  MCK(m->gerr.ensure(sizeof(int)));
-  MCK(cudaMemset(m->gerr.p, 0, sizeof(int)));
   const int din[kLayers] = {m->nip, kHidden, kHidden, kHidden};
   const int dout[kLayers] = {kHidden, kHidden, kHidden, kOutPad};
   for (int l = 0; l < kLayers; l++) {
     m->din[l] = din[l];
     m->dout[l] = dout[l];
-    const size_t nw = wcount(m, l);
-    for (DBuf *d : {&m->w[l], &m->mw[l], &m->vw[l], &m->gw[l]}) MCK(d->ensure(nw * 4));
-    for (DBuf *d : {&m->wb[l], &m->wbt[l]}) MCK(d->ensure(nw * 2));
-    for (DBuf *d : {&m->b[l], &m->mb[l], &m->vb[l], &m->gb[l]}) MCK(d->ensure(dout[l] * 4));
-    MCK(cudaMemset(m->mw[l].p, 0, nw * 4));
-    MCK(cudaMemset(m->vw[l].p, 0, nw * 4));
-    MCK(cudaMemset(m->b[l].p, 0, dout[l] * 4));
-    MCK(cudaMemset(m->mb[l].p, 0, dout[l] * 4));
-    MCK(cudaMemset(m->vb[l].p, 0, dout[l] * 4));
   }
-  MCK(m->fmean.ensure(m->nip * 4));
-  MCK(m->fistd.ensure(m->nip * 4));
-  MCK(m->tmean.ensure(kOut * 4));
-  MCK(m->tstd.ensure(kOut * 4));
+  Arena a;
+  DBuf *const flat[4][2] = {{m->gw, m->gb}, {m->w, m->b}, {m->mw, m->mb}, {m->vw, m->vb}};
+  for (auto &k : flat) {
+    for (int l = 0; l < kLayers; l++) {
+      a.add(k[0][l], wcount(m, l) * 4);
+      a.add(k[1][l], dout[l] * 4);
+    }
+    if (!m->flat) m->flat = (long long)(a.total / 4);
+  }
+  for (int l = 0; l < kLayers; l++) {
+    a.add(m->wb[l], wcount(m, l) * 2);
+    a.add(m->wbt[l], wcount(m, l) * 2);
+  }
+  a.add(m->fmean, m->nip * 4);
+  a.add(m->fistd, m->nip * 4);
+  a.add(m->tmean, kOut * 4);
+  a.add(m->tstd, kOut * 4);
+  a.add(m->tistd, kOut * 4);
+  a.add(m->gerr, sizeof(int));
+  a.add(m->loss, sizeof(double));
+  MCK(m->model.ensure(a.total));
+  a.place(m->model.p);
+  MCK(cudaMemset(m->model.p, 0, a.total));
   m->h_fmean.assign(m->nip, 0.f);
   m->h_fistd.assign(m->nip, 1.f);
   m->h_tmean.assign(kOut, 0.f);
@@ -1348,7 +1762,7 @@ void forward(me_mlp *m, int B, bool keep, cudaStream_t st) {
   }
 }
 
-// backward from dY (m->dyb, BF16 [B][32]) into m->gw / m->gb
+// backward from dY (m->dyb, BF16 [B][32]), added into m->gw / m->gb
 void backward(me_mlp *m, int B, cudaStream_t st) {
   const bf16 *dcur = m->dyb.as<bf16>();  // dZ of layer l, BF16 [B][dout]
   for (int l = kLayers - 1; l >= 0; l--) {
@@ -1361,9 +1775,7 @@ void backward(me_mlp *m, int B, cudaStream_t st) {
     transpose(aprev, B, din, aprevt, st);
     int split = 1;
     while (split < 16 && B % (2 * split * kTK) == 0 && B / (2 * split) >= 256) split *= 2;
-    cudaMemsetAsync(m->gw[l].p, 0, wcount(m, l) * 4, st);
     gemm(ctx(m), dzt, aprevt, dout, din, B, nullptr, nullptr, 0, nullptr, m->gw[l].as<float>(), st, split);
-    cudaMemsetAsync(m->gb[l].p, 0, dout * 4, st);
     const int chunk = 256;
     bias_grad_kernel<<<dim3((dout + 31) / 32, (B + chunk - 1) / chunk), dim3(32, 8), 0, st>>>(
         dcur, B, dout, chunk, m->gb[l].as<float>());
@@ -1382,17 +1794,73 @@ void adam_step(me_mlp *m, float lr, cudaStream_t st) {
   m->adam_t++;
   const float c1 = (float)(1.0 / (1.0 - pow((double)b1, (double)m->adam_t)));
   const float c2 = (float)(1.0 / (1.0 - pow((double)b2, (double)m->adam_t)));
+  AdamNet net;
+  net.w = m->w[0].as<float>();
+  net.m = m->mw[0].as<float>();
+  net.v = m->vw[0].as<float>();
+  net.g = m->gw[0].as<float>();
+  net.n = m->flat;
   for (int l = 0; l < kLayers; l++) {
-    const long long nw = (long long)wcount(m, l);
-    adam_kernel<<<nblk(nw), 256, 0, st>>>(m->w[l].as<float>(), m->mw[l].as<float>(),
-                                           m->vw[l].as<float>(), m->gw[l].as<float>(), nw,
-                                           m->din[l], lr, b1, b2, eps, c1, c2,
-                                           m->wb[l].as<bf16>(), m->wbt[l].as<bf16>(), m->dout[l]);
-    adam_kernel<<<nblk(m->dout[l]), 256, 0, st>>>(m->b[l].as<float>(), m->mb[l].as<float>(),
-                                                   m->vb[l].as<float>(), m->gb[l].as<float>(),
-                                                   m->dout[l], m->dout[l], lr, b1, b2, eps, c1,
-                                                   c2, nullptr, nullptr, 1);
+    net.off[l] = m->w[l].as<float>() - net.w;
+    net.rows[l] = m->dout[l];
+    net.cols[l] = m->din[l];
+    net.wb[l] = m->wb[l].as<bf16>();
+    net.wbt[l] = m->wbt[l].as<bf16>();
   }
+  adam_kernel<<<nblk(m->flat), 256, 0, st>>>(net, lr, b1, b2, eps, c1, c2);
+}
+
+// The gradients of B rows in two kernels, where the tcgen05 kernels are chosen
+// and can run (ok): the arguments of both, set up once for all steps.
+struct StepPlan {
+  bool ok = false;
+  StepMaps maps;
+  StepNet net;
+  GradMaps gmaps;
+  GradNet gnet;
+  unsigned tiles = 0, split = 1;
+};
+
+bool step_fused(const me_mlp *m) {
+  return m->gemm_path == GemmPath::tcgen05 && device_facts().step_ok;
+}
+
+void plan_step(me_mlp *m, int B, StepPlan *p) {
+  memset(&p->maps, 0, sizeof(p->maps));
+  for (int l = 0; l < kLayers; l++) {
+    const bf16 *in = l ? m->sat[l - 1].as<bf16>() : m->sxt.as<bf16>();
+    if (!cached_tile_map(&m->maps, &p->maps.w[l], m->wb[l].as<bf16>(), m->dout[l], m->din[l],
+                         l < kLayers - 1 ? 128 : kOutPad) ||
+        (l > 0 && !cached_tile_map(&m->maps, &p->maps.t[l], m->wbt[l].as<bf16>(), m->din[l],
+                                   m->dout[l], 128)) ||
+        !cached_tile_map(&m->maps, &p->gmaps.a[l], m->sdzt[l].as<bf16>(), m->dout[l], B,
+                         me::umma::kBM) ||
+        !cached_tile_map(&m->maps, &p->gmaps.b[l], in, m->din[l], B, kGradN))
+      return;
+    p->net.bias[l] = m->b[l].as<float>();
+    if (l < kLayers - 1) p->net.at[l] = m->sat[l].as<bf16>();
+    p->net.dzt[l] = m->sdzt[l].as<bf16>();
+    p->net.gb[l] = m->gb[l].as<float>();
+    p->gnet.gw[l] = m->gw[l].as<float>();
+    p->gnet.m[l] = m->dout[l];
+    p->gnet.n[l] = m->din[l];
+    p->gnet.tiles[l] = ((m->dout[l] + me::umma::kBM - 1) / me::umma::kBM) *
+                       ((m->din[l] + kGradN - 1) / kGradN);
+    p->tiles += (unsigned)p->gnet.tiles[l];
+  }
+  p->net.xt = m->sxt.as<bf16>();
+  while (p->split < 16 && B / (2 * p->split) >= 256) p->split *= 2;
+  while (B % (p->split * me::umma::kBK)) p->split /= 2;  // (B % 256 == 0: ends at 4 or before)
+  p->ok = true;
+}
+
+void run_step(me_mlp *m, const StepPlan &p, int B, const bf16 *X, const float *T,
+              const long long *idx, cudaStream_t st) {
+  mlp_step_kernel<<<B / kStepRows, kStepThreads, kStepSmem, st>>>(
+      p.maps, p.net, X, idx, T, B, m->nip, m->loss.as<double>(), m->gerr.as<int>());
+  mlp_wgrad_kernel<<<dim3(p.tiles, p.split), 128, me::umma::smem_bytes(kGradN), st>>>(
+      p.gmaps, p.gnet, B, m->gerr.as<int>());
+  m->gemm_launches[(int)GemmPath::tcgen05] += kLayers + 2 * kLayers - 1;
 }
 
 // loss and gradients of the rows idx[0..B) of the standardised targets T
@@ -1512,18 +1980,23 @@ extern "C" int me_mlp_train(me_plan *plan, const me_mlp_train_params *tp, me_mlp
   const long long n = tp->samples;
   const int nip = m->nip;
   // ---- training set: FP32 synthesis on the plan's grid, then standardisation ----
-  DBuf Xf, X, T;
+  DBuf Xf, set, X, T;
   MCK(Xf.ensure((size_t)n * nip * 4));
-  MCK(T.ensure((size_t)n * kOut * 4));
+  Arena parts;
+  parts.add(X, (size_t)n * nip * 2);
+  parts.add(T, (size_t)n * kOut * 4);
+  MCK(set.ensure(parts.total));
+  parts.place(set.p);
   Prior pr;
   prior_from(tp, pr);
   synth_train_kernel<<<nblk(n, 128), 128, 0, st>>>(P, pr, tp->seed, n, nip, Xf.as<float>(),
                                                     T.as<float>());
   MCK(cudaGetLastError());
   {
+    // the sums lie in X until the features take their place (n >= 256)
     DBuf s1, s2;
-    MCK(s1.ensure(nip * 8));
-    MCK(s2.ensure(nip * 8));
+    s1.view(X.p, nip * 8);
+    s2.view(X.as<double>() + nip, nip * 8);
     std::vector<double> a(nip), b(nip);
     moments_kernel<<<nip, 256, 0, st>>>(Xf.as<float>(), n, nip, s1.as<double>(), s2.as<double>());
     MCK(cudaMemcpy(a.data(), s1.p, nip * 8, cudaMemcpyDeviceToHost));
@@ -1545,23 +2018,34 @@ extern "C" int me_mlp_train(me_plan *plan, const me_mlp_train_params *tp, me_mlp
     }
     rc = upload_standardisation(m);
     if (rc) return rc;
-    DBuf tiv;
-    MCK(tiv.ensure(kOut * 4));
-    MCK(cudaMemcpy(tiv.p, tinv.data(), kOut * 4, cudaMemcpyHostToDevice));
-    MCK(X.ensure((size_t)n * nip * 2));
+    MCK(cudaMemcpy(m->tistd.p, tinv.data(), kOut * 4, cudaMemcpyHostToDevice));
     standardise_kernel<<<nblk((long long)n * nip), 256, 0, st>>>(
         Xf.as<float>(), n, nip, m->fmean.as<float>(), m->fistd.as<float>(), X.as<bf16>());
     standardise_kernel<<<nblk((long long)n * kOut), 256, 0, st>>>(
-        T.as<float>(), n, kOut, m->tmean.as<float>(), tiv.as<float>(), nullptr);
-    MCK(cudaStreamSynchronize(st));
+        T.as<float>(), n, kOut, m->tmean.as<float>(), m->tistd.as<float>(), nullptr);
+    MCK(cudaGetLastError());
   }
-  Xf.release();
   // ---- Adam on shuffled batches ----
+  // What follows lies where the FP32 features were, if it fits there; they are
+  // not needed any more.
   const int B = tp->batch;
-  rc = ensure_batch(m, B);
-  if (rc) return rc;
   DBuf perm;
-  MCK(perm.ensure((size_t)n * sizeof(long long)));
+  const size_t permb = ((size_t)n * sizeof(long long) + 255) / 256 * 256;  // <= Xf (nip >= 32)
+  StepPlan sp;
+  if (step_fused(m)) {
+    perm.view(Xf.p, permb);
+    rc = ensure_step(m, B, Xf.as<char>() + permb, Xf.n - permb);
+    if (rc) return rc;
+    plan_step(m, B, &sp);
+  }
+  if (!sp.ok) {
+    MCK(cudaStreamSynchronize(st));
+    Xf.release();
+    rc = ensure_batch(m, B);
+    if (rc) return rc;
+    perm.view(nullptr, 0);
+    MCK(perm.ensure((size_t)n * sizeof(long long)));
+  }
   int bits = 1;
   while ((1LL << bits) < n) bits++;
   const long long steps = n / B;
@@ -1573,9 +2057,13 @@ extern "C" int me_mlp_train(me_plan *plan, const me_mlp_train_params *tp, me_mlp
     MCK(cudaMemsetAsync(m->loss.p, 0, sizeof(double), st));
     for (long long s = 0; s < steps; s++) {
       const long long *idx = perm.as<long long>() + s * B;
-      gather_kernel<<<nblk((long long)B * nip), 256, 0, st>>>(X.as<bf16>(), idx, B, nip,
-                                                              m->xb.as<bf16>());
-      loss_grad(m, B, T.as<float>(), idx, st);
+      if (sp.ok) {
+        run_step(m, sp, B, X.as<bf16>(), T.as<float>(), idx, st);
+      } else {
+        gather_kernel<<<nblk((long long)B * nip), 256, 0, st>>>(X.as<bf16>(), idx, B, nip,
+                                                                m->xb.as<bf16>());
+        loss_grad(m, B, T.as<float>(), idx, st);
+      }
       adam_step(m, (float)tp->lr, st);
     }
     MCK(cudaGetLastError());
@@ -1585,6 +2073,12 @@ extern "C" int me_mlp_train(me_plan *plan, const me_mlp_train_params *tp, me_mlp
     rc = gemm_status(m);
     if (rc) return rc;
     last = l / (double)steps;
+  }
+  // (what lay in the training set's memory goes with it)
+  if (m->step_cap == 0) {
+    m->sxt.release();
+    for (DBuf &d : m->sat) d.release();
+    for (DBuf &d : m->sdzt) d.release();
   }
   if (final_loss) *final_loss = last;
   *out = guard.release();
@@ -1618,7 +2112,7 @@ static bool predict_fused(me_mlp *m, const double *d_prof, long npix, double *d_
     go(mlp_predict_kernel<true>);
   else
     go(mlp_predict_kernel<false>);
-  m->gemm_launches[(int)GemmPath::tcgen05]++;
+  m->gemm_launches[(int)GemmPath::tcgen05] += kLayers;
   return true;
 }
 
@@ -1742,7 +2236,17 @@ extern "C" int me_mlp_loss_grad(me_mlp *m, const float *x, const float *t, int r
                                                                m->xb.as<bf16>());
   iota_kernel<<<nblk(rows), 256>>>(idx.as<long long>(), rows);
   MCK(cudaMemset(m->loss.p, 0, sizeof(double)));
-  loss_grad(m, rows, tf.as<float>(), idx.as<long long>(), nullptr);
+  MCK(cudaMemset(m->gw[0].p, 0, (size_t)m->flat * 4));
+  StepPlan sp;
+  if (step_fused(m)) {
+    rc = ensure_step(m, rows, nullptr, 0);
+    if (rc) return rc;
+    plan_step(m, rows, &sp);
+  }
+  if (sp.ok)
+    run_step(m, sp, rows, m->xb.as<bf16>(), tf.as<float>(), idx.as<long long>(), nullptr);
+  else
+    loss_grad(m, rows, tf.as<float>(), idx.as<long long>(), nullptr);
   MCK(cudaGetLastError());
   MCK(cudaDeviceSynchronize());
   rc = gemm_status(m);
