@@ -502,11 +502,18 @@ __device__ __forceinline__ float feature_value(int s, float v, float imax_inv) {
   return s == 0 ? v * imax_inv - 1.f : 10.f * v * imax_inv;
 }
 
+// The training set leaves the synthesis in tiles of 128 samples, each value of a
+// tile's samples side by side ([tile][column][128]): a thread makes a sample, so
+// a warp's stores and the pass back over the profile are contiguous.  131,072
+// samples of 60 wavelengths: 212 us, in rows 571; the moments of the features
+// and targets and their standardisation (transposed in shared memory) 111, 349.
+constexpr int kTile = 128;
+
 __global__ void synth_train_kernel(const __grid_constant__ DevPlan P, Prior pr,
                                    unsigned long long seed, long long n, int ld, float *Xraw,
                                    float *Tgt) {
   __shared__ float s_tab[100];
-  __shared__ float s_rden[kRden * 128];
+  __shared__ float s_rden[kRden * kTile];
   VoigtK<float> K;
   voigt_block_setup<float>(K, P, s_tab);
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -532,7 +539,8 @@ __global__ void synth_train_kernel(const __grid_constant__ DevPlan P, Prior pr,
   voigt_prepare<float>(K, c.p5, s_rden + threadIdx.x, blockDim.x);
   const float ones[4] = {1.f, 1.f, 1.f, 1.f};
   const int nl = P.nl;
-  float *xr = Xraw + (size_t)i * ld;  // row of this sample: the profile, then features
+  // this sample's column of its tile: the profile, then the features
+  float *xr = Xraw + (size_t)blockIdx.x * ld * kTile + threadIdx.x;
   float imax = 0.f;
   unsigned long long nseed = seed ^ 0x9E3779B97F4A7C15ull;
   for (int iw = 0; iw < nl; iw++) {
@@ -556,60 +564,96 @@ __global__ void synth_train_kernel(const __grid_constant__ DevPlan P, Prior pr,
       syn[s + 1] += pr.noise * r * sn;
     }
 #pragma unroll
-    for (int s = 0; s < 4; s++) xr[s * nl + iw] = syn[s];
+    for (int s = 0; s < 4; s++) xr[(size_t)(s * nl + iw) * kTile] = syn[s];
     imax = fmaxf(imax, syn[0]);
   }
   const float inv = 1.f / imax;
-  for (int k = 0; k < 4 * nl; k++) xr[k] = feature_value(k / nl, xr[k], inv);
-  for (int k = 4 * nl; k < ld; k++) xr[k] = 0.f;
-  float *t = Tgt + (size_t)i * kOut;
-  t[0] = (float)par[0];
-  t[1] = (float)cost;
-  t[2] = (float)sin(2.0 * par[2]);
-  t[3] = (float)cos(2.0 * par[2]);
-  t[4] = (float)par[3];
-  t[5] = (float)par[4];
-  t[6] = (float)par[5];
-  t[7] = (float)par[6];
-  t[8] = (float)par[8];
-  t[9] = (float)(par[7] * inv);
+  for (int k = 0; k < 4 * nl; k++) {
+    float *x = xr + (size_t)k * kTile;
+    *x = feature_value(k < nl ? 0 : 1, *x, inv);
+  }
+  for (int k = 4 * nl; k < ld; k++) xr[(size_t)k * kTile] = 0.f;
+  float *t = Tgt + (size_t)blockIdx.x * kOut * kTile + threadIdx.x;
+  t[0 * kTile] = (float)par[0];
+  t[1 * kTile] = (float)cost;
+  t[2 * kTile] = (float)sin(2.0 * par[2]);
+  t[3 * kTile] = (float)cos(2.0 * par[2]);
+  t[4 * kTile] = (float)par[3];
+  t[5 * kTile] = (float)par[4];
+  t[6 * kTile] = (float)par[5];
+  t[7 * kTile] = (float)par[6];
+  t[8 * kTile] = (float)par[8];
+  t[9 * kTile] = (float)(par[7] * inv);
 }
 
-// per-column mean and 1/std over n rows of an FP32 [n][cols] array
-__global__ void moments_kernel(const float *x, long long n, int cols, double *sum, double *sum2) {
-  const int col = blockIdx.x;
+// Sums and sums of squares of the columns of n tiled samples, in FP64: a warp
+// per column and share of the tiles into part [gridDim.y][cols][2], added up in
+// order by moments_sum_kernel.
+__global__ void moments_kernel(const float *x, long long n, int cols, double *part) {
+  const int col = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x & 31;
+  if (col >= cols) return;
   double s = 0, s2 = 0;
-  for (long long r = threadIdx.x; r < n; r += blockDim.x) {
-    const double v = x[(size_t)r * cols + col];
-    s += v;
-    s2 += v * v;
+  for (long long t = blockIdx.y; t * kTile < n; t += gridDim.y) {
+    const float4 f = __ldg(reinterpret_cast<const float4 *>(
+        x + ((size_t)t * cols + col) * kTile + lane * 4));
+    const double v[4] = {f.x, f.y, f.z, f.w};
+#pragma unroll
+    for (int e = 0; e < 4; e++)
+      if (t * kTile + lane * 4 + e < n) {
+        s += v[e];
+        s2 += v[e] * v[e];
+      }
   }
-  __shared__ double a[256], b[256];
-  a[threadIdx.x] = s;
-  b[threadIdx.x] = s2;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) {
-      a[threadIdx.x] += a[threadIdx.x + w];
-      b[threadIdx.x] += b[threadIdx.x + w];
-    }
-    __syncthreads();
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    s += __shfl_xor_sync(0xffffffffu, s, o);
+    s2 += __shfl_xor_sync(0xffffffffu, s2, o);
   }
-  if (threadIdx.x == 0) {
-    sum[col] = a[0];
-    sum2[col] = b[0];
+  if (lane == 0) {
+    part[((size_t)blockIdx.y * cols + col) * 2] = s;
+    part[((size_t)blockIdx.y * cols + col) * 2 + 1] = s2;
   }
 }
 
-// x <- (x - mean) * istd, written to BF16 X (and in place to the FP32 copy)
-__global__ void standardise_kernel(float *xf, long long n, int cols, const float *mean,
-                                   const float *istd, bf16 *X) {
+__global__ void moments_sum_kernel(const double *part, int shares, int cols, double *sum) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= 2 * cols) return;
+  double s = 0;
+  for (int k = 0; k < shares; k++) s += part[(size_t)k * 2 * cols + i];
+  sum[i] = s;
+}
+
+// (x - mean) * istd of tiled samples, 32 columns of a tile per CTA, as the BF16
+// rows X [n][cols] (cols % 32 == 0)
+__global__ void __launch_bounds__(256)
+    standardise_kernel(const float *x, long long n, int cols, const float *mean,
+                       const float *istd, bf16 *X) {
+  __shared__ __nv_bfloat162 s_out[kTile][17];
+  const int c0 = blockIdx.y * 32;
+  for (int i = threadIdx.x; i < 16 * kTile; i += 256) {
+    const int c = c0 + 2 * (i / kTile), r = i % kTile;
+    const float *p = x + ((size_t)blockIdx.x * cols + c) * kTile + r;
+    s_out[r][i / kTile] = __floats2bfloat162_rn((__ldg(p) - __ldg(mean + c)) * __ldg(istd + c),
+                                                (__ldg(p + kTile) - __ldg(mean + c + 1)) *
+                                                    __ldg(istd + c + 1));
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 16 * kTile; i += 256) {
+    const long long r = (long long)blockIdx.x * kTile + i / 16;
+    if (r < n)
+      *reinterpret_cast<__nv_bfloat162 *>(X + (size_t)r * cols + c0 + 2 * (i % 16)) =
+          s_out[i / 16][i % 16];
+  }
+}
+
+// the same of tiled targets, as FP32 rows [n][kOut]
+__global__ void standardise_targets_kernel(const float *x, long long n, const float *mean,
+                                           const float *istd, float *T) {
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= n * cols) return;
-  const int c = (int)(i % cols);
-  const float v = (xf[i] - mean[c]) * istd[c];
-  xf[i] = v;
-  if (X) X[i] = __float2bfloat16(v);
+  if (i >= n) return;
+  const float *p = x + (size_t)(i / kTile) * kOut * kTile + i % kTile;
+#pragma unroll
+  for (int k = 0; k < kOut; k++) T[(size_t)i * kOut + k] = (p[k * kTile] - mean[k]) * istd[k];
 }
 
 // features of map profiles (FP64 [n][4][nl]) for inference, standardised:
@@ -1981,37 +2025,43 @@ extern "C" int me_mlp_train(me_plan *plan, const me_mlp_train_params *tp, me_mlp
   const int nip = m->nip;
   // ---- training set: FP32 synthesis on the plan's grid, then standardisation ----
   DBuf Xf, set, X, T;
-  MCK(Xf.ensure((size_t)n * nip * 4));
+  const size_t tiles = (size_t)((n + kTile - 1) / kTile);
   Arena parts;
+  if (step_fused(m))  // (the other path gives the FP32 features back before its buffers)
+    parts.add(Xf, tiles * kTile * nip * 4);
+  else
+    MCK(Xf.ensure(tiles * kTile * nip * 4));
   parts.add(X, (size_t)n * nip * 2);
   parts.add(T, (size_t)n * kOut * 4);
   MCK(set.ensure(parts.total));
   parts.place(set.p);
   Prior pr;
   prior_from(tp, pr);
-  synth_train_kernel<<<nblk(n, 128), 128, 0, st>>>(P, pr, tp->seed, n, nip, Xf.as<float>(),
-                                                    T.as<float>());
+  // The targets lie in X until the features take their place (n >= 256, so 64 n
+  // bytes and more hold the tiles), the sums in the gradients.
+  float *const traw = X.as<float>();
+  synth_train_kernel<<<(unsigned)tiles, kTile, 0, st>>>(P, pr, tp->seed, n, nip, Xf.as<float>(),
+                                                        traw);
   MCK(cudaGetLastError());
   {
-    // the sums lie in X until the features take their place (n >= 256)
-    DBuf s1, s2;
-    s1.view(X.p, nip * 8);
-    s2.view(X.as<double>() + nip, nip * 8);
-    std::vector<double> a(nip), b(nip);
-    moments_kernel<<<nip, 256, 0, st>>>(Xf.as<float>(), n, nip, s1.as<double>(), s2.as<double>());
-    MCK(cudaMemcpy(a.data(), s1.p, nip * 8, cudaMemcpyDeviceToHost));
-    MCK(cudaMemcpy(b.data(), s2.p, nip * 8, cudaMemcpyDeviceToHost));
+    const int shares = (int)(tiles < 64 ? tiles : 64);
+    double *const sums = m->gw[0].as<double>(), *const part = sums + 2 * nip;
+    std::vector<double> a(2 * nip);
+    auto moments = [&](const float *x, int cols) {
+      moments_kernel<<<dim3((cols + 7) / 8, shares), 256, 0, st>>>(x, n, cols, part);
+      moments_sum_kernel<<<nblk(2 * cols), 256, 0, st>>>(part, shares, cols, sums);
+      return cudaMemcpy(a.data(), sums, 2 * cols * 8, cudaMemcpyDeviceToHost);
+    };
+    MCK(moments(Xf.as<float>(), nip));
     for (int c = 0; c < nip; c++) {
-      const double mu = a[c] / n, var = b[c] / n - mu * mu;
+      const double mu = a[2 * c] / n, var = a[2 * c + 1] / n - mu * mu;
       m->h_fmean[c] = c < m->nin ? (float)mu : 0.f;
       m->h_fistd[c] = (c < m->nin && var > 1e-20) ? (float)(1.0 / sqrt(var)) : 0.f;
     }
-    moments_kernel<<<kOut, 256, 0, st>>>(T.as<float>(), n, kOut, s1.as<double>(), s2.as<double>());
-    MCK(cudaMemcpy(a.data(), s1.p, kOut * 8, cudaMemcpyDeviceToHost));
-    MCK(cudaMemcpy(b.data(), s2.p, kOut * 8, cudaMemcpyDeviceToHost));
+    MCK(moments(traw, kOut));
     std::vector<float> tinv(kOut);
     for (int c = 0; c < kOut; c++) {
-      const double mu = a[c] / n, var = b[c] / n - mu * mu;
+      const double mu = a[2 * c] / n, var = a[2 * c + 1] / n - mu * mu;
       m->h_tmean[c] = (float)mu;
       m->h_tstd[c] = var > 1e-20 ? (float)sqrt(var) : 1.f;
       tinv[c] = 1.f / m->h_tstd[c];
@@ -2019,10 +2069,11 @@ extern "C" int me_mlp_train(me_plan *plan, const me_mlp_train_params *tp, me_mlp
     rc = upload_standardisation(m);
     if (rc) return rc;
     MCK(cudaMemcpy(m->tistd.p, tinv.data(), kOut * 4, cudaMemcpyHostToDevice));
-    standardise_kernel<<<nblk((long long)n * nip), 256, 0, st>>>(
+    standardise_targets_kernel<<<nblk(n), 256, 0, st>>>(traw, n, m->tmean.as<float>(),
+                                                        m->tistd.as<float>(), T.as<float>());
+    standardise_kernel<<<dim3((unsigned)tiles, nip / 32), 256, 0, st>>>(
         Xf.as<float>(), n, nip, m->fmean.as<float>(), m->fistd.as<float>(), X.as<bf16>());
-    standardise_kernel<<<nblk((long long)n * kOut), 256, 0, st>>>(
-        T.as<float>(), n, kOut, m->tmean.as<float>(), m->tistd.as<float>(), nullptr);
+    MCK(cudaMemsetAsync(m->gw[0].p, 0, (size_t)m->flat * 4, st));
     MCK(cudaGetLastError());
   }
   // ---- Adam on shuffled batches ----
@@ -2181,22 +2232,16 @@ extern "C" int me_mlp_shape(const me_mlp *m, int *nl, int *nin_pad, long long *n
 }
 
 namespace {
-// copies the parameters (or gradients) between a flat host array and the device
+// copies the parameters (or gradients) between a flat host array and the
+// device, where they lie in the same order without gaps (alloc_model: every
+// layer's sizes but the last bias's are multiples of 64 floats)
 int copy_flat(const me_mlp *m, bool grads, float *host, bool to_host) {
-  size_t off = 0;
-  for (int l = 0; l < kLayers; l++) {
-    const DBuf &W = grads ? m->gw[l] : m->w[l];
-    const DBuf &Bv = grads ? m->gb[l] : m->b[l];
-    const size_t nw = wcount(m, l);
-    if (to_host) {
-      MCK(cudaMemcpy(host + off, W.p, nw * 4, cudaMemcpyDeviceToHost));
-      MCK(cudaMemcpy(host + off + nw, Bv.p, m->dout[l] * 4, cudaMemcpyDeviceToHost));
-    } else {
-      MCK(cudaMemcpy(W.p, host + off, nw * 4, cudaMemcpyHostToDevice));
-      MCK(cudaMemcpy(Bv.p, host + off + nw, m->dout[l] * 4, cudaMemcpyHostToDevice));
-    }
-    off += nw + m->dout[l];
-  }
+  void *dev = grads ? m->gw[0].p : m->w[0].p;
+  const size_t bytes = (size_t)param_count(m) * 4;
+  if (to_host)
+    MCK(cudaMemcpy(host, dev, bytes, cudaMemcpyDeviceToHost));
+  else
+    MCK(cudaMemcpy(dev, host, bytes, cudaMemcpyHostToDevice));
   return ME_OK;
 }
 }  // namespace
