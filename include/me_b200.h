@@ -188,11 +188,11 @@ int me_plan_window(const me_plan *plan);
 void me_plan_set_window(me_plan *plan, int window);
 
 /* Pixels in flight at or below which, once every pixel of a batch has been
- * taken from the queue, the remaining ones are run to the end one warp per
- * pixel (their synthesis spread over the lanes) instead of one LM step per
- * launch round: the same arithmetic up to the compiler's contraction of
- * multiply-adds, and a much shorter tail.  -1 (default): half a wave of the
- * tail kernel's warps on this device (~900 on a B200); 0: rounds only. */
+ * taken from the queue, the remaining ones are run to the end one CTA per
+ * pixel (one warp on FP64 plans; their synthesis spread over the lanes)
+ * instead of one LM step per launch round: the same arithmetic up to the
+ * compiler's contraction of multiply-adds, and a much shorter tail.  -1
+ * (default): four per SM of this device (592 on a B200); 0: rounds only. */
 int me_plan_tail_slots(const me_plan *plan);
 /* Once every pixel of a batch has been taken from the queue, the LM rounds
  * give each pixel still in flight a group of lanes (2, 4, ... up to this
@@ -213,8 +213,8 @@ int me_plan_svd_lanes(const me_plan *plan);
 int me_plan_svd_registers(const me_plan *plan);
 void me_plan_set_svd_registers(me_plan *plan, int mode);
 /* The LM rounds between two checks of the queue go to the GPU as one CUDA
- * graph, captured once per batch for each lane-group size (default on; off:
- * one launch per kernel).  Profiling (me_plan_set_profiling) launches
+ * graph, captured once per batch for each lane-group size that runs long
+ * enough to repay it (default on; off: one launch per kernel always).  Profiling (me_plan_set_profiling) launches
  * directly. */
 void me_plan_set_graphs(me_plan *plan, int on);
 /* The SVD solves of trials after a rejection run on a second stream beside

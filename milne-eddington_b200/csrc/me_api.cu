@@ -703,8 +703,9 @@ void trace_poll(me_plan *p, long long rounds, long long next, int busy, int grou
 
 // Runs one queue (A.count items) to completion: rounds of jac_kernel,
 // svd_kernel and trial_kernel on the plan's slots while the queue feeds them,
-// then, once it is empty and at most tail_slots pixels remain, finish_kernel
-// (one warp per pixel, no per-round launches) for the rest.
+// then, once it is empty and at most tail_slots pixels remain, tail_kernel (one
+// CTA per pixel; FP64 plans: finish_kernel, one warp) for the rest, without
+// per-round launches.
 int run_queue(me_plan *p, const me::InvertArgs &A, cudaStream_t st, long long &rounds,
               cudaEvent_t feed_done = nullptr) {
   const long long cap = p->window > 0 ? p->window : 131072;
@@ -730,11 +731,18 @@ int run_queue(me_plan *p, const me::InvertArgs &A, cudaStream_t st, long long &r
   // 1..5 lane groups of 2..32; they hold this queue's arguments, so they live
   // for this call only
   cudaGraphExec_t graphs[6] = {};
-  // a group size's first rounds in this queue run as direct launches, so
-  // that every kernel a graph holds has run (and been loaded) before its
-  // capture; a capture that fails all the same falls back to direct launches
-  // for the rest of the queue
-  bool ran_direct[6] = {};
+  // A group size's first kGraphAfter batches of rounds in this queue run as
+  // direct launches.  Capturing, instantiating and destroying a graph costs
+  // some 0.6 ms, and a launch of it saves a batch nothing that shows: 1 M
+  // pixels (7 batches of full rounds, 62 of lane groups in five sizes) took
+  // 136.5 ms with a graph from the second batch of each size on and 132.9
+  // directly, 50 k with restarts 82.6 and 80.0; 4 M pixels 383.6 and 382.2.
+  // Beyond some thirty batches the cost no longer shows, and one launch in
+  // place of fifty leaves the host free.  Every kernel a graph holds has then
+  // run (and been loaded) before its capture; a capture that fails all the
+  // same falls back to direct launches for the rest of the queue.
+  constexpr int kGraphAfter = 32;
+  int direct[6] = {};
   bool graphs_ok = true;
   auto group_index = [](int g) {
     int i = 0;
@@ -785,10 +793,10 @@ int run_queue(me_plan *p, const me::InvertArgs &A, cudaStream_t st, long long &r
     const int gi = group_index(group);
     const int nr = group > 1 ? p->drain_poll : p->poll_rounds;
     cudaGraphExec_t *gx =
-        (graphs_ok && ran_direct[gi] && p->use_graphs && !p->profile && nr % 2 == 0)
+        (graphs_ok && direct[gi] >= kGraphAfter && p->use_graphs && !p->profile && nr % 2 == 0)
             ? &graphs[gi]
             : nullptr;
-    ran_direct[gi] = true;
+    if (!gx) direct[gi]++;
     if (gx && !*gx) {
       cudaGraph_t g = nullptr;
       CK(cudaStreamBeginCapture(p->stream, cudaStreamCaptureModeThreadLocal));
