@@ -24,7 +24,8 @@ namespace {
 // wavelengths.  One thread per pixel stored 8 bytes every 32 nl (288 nl with
 // the Jacobian) and left most of the device idle on maps of a few thousand
 // pixels.
-// flags (nullable): pixels without bit 0 get zeros instead.
+// flags (nullable): pixels without bit 0 get zeros instead; their parameters,
+// which nothing has written, are not read.
 // Measured on a B200, one thread per pixel against this: 262144 profiles of 60
 // wavelengths, FP32, 912 -> 288 us; 10007 FP64 Jacobians of 112 wavelengths 1600
 // -> 533 us; 37 FP32 Jacobians 147 -> 20 us (host call included).  The large FP32
@@ -38,6 +39,7 @@ struct SynthPixel {
   SynthCall<T> c;
   T yy, inv_y;
   T rden[sizeof(T) == sizeof(float) ? kRden : 1];
+  bool live;
 };
 
 enum SynthMode { kPlain, kFilter, kFilterSplit };  // no filter; with one: see launch_synth_t
@@ -55,19 +57,22 @@ __global__ void __launch_bounds__(kSynthThreads)
   if ((int)threadIdx.x < here) {
     SynthPixel<T> &o = s_px[threadIdx.x];
     const long long i = first + threadIdx.x;
-    double mp[9], step[9];
+    o.live = !flags || (flags[i] & 1);
+    if (o.live) {
+      double mp[9], step[9];
 #pragma unroll
-    for (int k = 0; k < 9; k++) {
-      mp[k] = par[i * 9 + k];
-      step[k] = P.step[k];
+      for (int k = 0; k < 9; k++) {
+        mp[k] = par[i * 9 + k];
+        step[k] = P.step[k];
+      }
+      step[7] = step7;
+      SynthCall<T> c;
+      synth_setup<T>(c, mp, P, step);
+      voigt_prepare<T>(K, c.p5, o.rden, 1);
+      o.c = c;
+      o.yy = K.yy;
+      o.inv_y = K.inv_y;
     }
-    step[7] = step7;
-    SynthCall<T> c;
-    synth_setup<T>(c, mp, P, step);
-    voigt_prepare<T>(K, c.p5, o.rden, 1);
-    o.c = c;
-    o.yy = K.yy;
-    o.inv_y = K.inv_y;
   }
   __syncthreads();
   const int nl = P.nl;
@@ -84,8 +89,8 @@ __global__ void __launch_bounds__(kSynthThreads)
     const int ns = P.nsub, tid = threadIdx.x, total = here * nl * ns;
     for (int p0 = 0; p0 < total; p0 += kSynthThreads) {
       const int e = p0 + tid;
-      if (e < total) {
-        const int p = e / (nl * ns);
+      const int p = e < total ? e / (nl * ns) : 0;
+      if (e < total && s_px[p].live) {
         const SynthPixel<T> &o = s_px[p];
         K.yy = o.yy;
         K.inv_y = o.inv_y;
@@ -111,16 +116,18 @@ __global__ void __launch_bounds__(kSynthThreads)
         const int q0 = w * ns > p0 ? w * ns : p0;
         const int q1 = (w + 1) * ns < p1 ? (w + 1) * ns : p1;
         T v = q0 == w * ns ? T(0) : s_part[m];
-        for (int q = q0; q < q1; q++) v += T(P.sub_w[q - w * ns]) * s_pt[(q - p0) * E + m];
+        if (s_px[w / nl].live)
+          for (int q = q0; q < q1; q++) v += T(P.sub_w[q - w * ns]) * s_pt[(q - p0) * E + m];
+        else
+          v = T(0);
         if (q1 < (w + 1) * ns) {
           carry = v;
           continue;
         }
         const size_t i = (size_t)(first + w / nl);
         const int iw = w % nl;
-        const bool live = !flags || (flags[i] & 1);
         if (m < 4)
-          prof[(i * 4 + m) * nl + iw] = live ? (double)v : 0.0;
+          prof[(i * 4 + m) * nl + iw] = (double)v;
         else
           jac[(i * 36 + m - 4) * nl + iw] = (double)v;
       }
@@ -138,7 +145,7 @@ __global__ void __launch_bounds__(kSynthThreads)
     const SynthPixel<T> &o = s_px[p];
     const size_t i = (size_t)(first + p);
     double *out = prof + i * 4 * nl + iw;
-    if (flags && !(flags[i] & 1)) {
+    if (!o.live) {
 #pragma unroll
       for (int s = 0; s < 4; s++) out[s * nl] = 0.0;
       continue;
