@@ -557,6 +557,12 @@ int me_mlp_set_gemm(me_mlp *mlp, int path);
  * launch of the fused inference or training kernels runs several). */
 int me_mlp_gemm_launches(const me_mlp *mlp, long long *tcgen05, long long *mma_sync);
 
+/* The waits inside the fused inference and training kernels, for testing how
+ * they end: each gives up after `tries` polls (0: the default), upon which the call that
+ * launched the kernel fails with ME_ERR_CUDA and the initialiser stays usable.  drop: events of which no waiting side learns: 0 none, 1 the loads of
+ * weights, 2 the completion of MMAs, 3 the release of stages. */
+int me_mlp_set_waits(me_mlp *mlp, unsigned tries, int drop);
+
 /* One GEMM of the initialiser's kernels, for testing them: with A [m][r] and
  * Bt [n][r] row-major BF16 bit patterns (host), z [m][n] = A Bt^T + bias
  * (bias [n] or NULL) and y [m][n] = GELU(z) if gelu else z, FP32 host

@@ -745,9 +745,12 @@ __global__ void decode_kernel(const float *Y, long long n, int ld, const float *
 //   1: 46, 45;  1,000: 53, 47;  18,900: 90, 50;  37,889: 162, 95;  300,007: 921, 493
 // and of 112: 1: 52, 51;  18,900: 106, 56;  75,000: 313, 163.  So it is used at
 // every count; the six launches remain for the mma.sync GEMMs.
-// Waits are bounded as in umma_gemm_kernel; after one runs out the CTA writes a
-// code to *err, stops loading and multiplying, keeps its barriers in step and
-// leaves its results unwritten.
+// Waits are bounded.  The first to run out writes a code to *err (1: weights, 2: a
+// free stage, 3: the accumulator) and raises the CTA's stop flag, at which all
+// other waits end too.  The named barriers have no limit: every warp passes each
+// of them once per phase with bar.sync, whatever its waits gave, so that none
+// runs ahead and none is left behind.  Results are then left unwritten, and the
+// CTA ends once its own copies have landed and its MMAs are done.
 // ---------------------------------------------------------------------------
 constexpr int kPredWarps = 8;  // per tile
 constexpr int kPredThreads = (2 * kPredWarps + 2) * 32;
@@ -756,13 +759,31 @@ constexpr int kPredBox = 128 * me::umma::kBK * 2;  // a box of weights
 constexpr int kPredStage = 2 * kPredBox;           // 64 inputs of a layer
 constexpr int kPredStages = 3;
 constexpr int kPredA = (kPredK / me::umma::kBK) * me::umma::kStageA;
-constexpr int kPredBars = 128;
+constexpr int kPredBars = 128;  // mbarriers, tensor-memory base, stop flag
 constexpr int kPredSmem = 2 * kPredA + kPredStages * kPredStage + kPredBars + 2 * 128 * 4;
 
 struct PredNet {
   const float *bias[kLayers];
   const float *fmean, *fistd, *tmean, *tstd;
 };
+
+// The limit of a kernel's waits and, for tests of what follows when one runs
+// out, a kind of event that arrives nowhere: a barrier's address is taken here,
+// once, so that it costs the loops nothing.
+struct WaitRules {
+  uint32_t tries = me::umma::kWaitTries;
+  int drop = 0;  // 1: the loads of weights, 2: the MMAs' completion, 3: the stages' release
+};
+
+// mbar_wait for a CTA's roles: false, with the error and the stop flag raised,
+// when it runs out.
+__device__ __forceinline__ bool role_wait(uint32_t bar, uint32_t parity, const WaitRules &rules,
+                                          volatile uint32_t *stop, int *err, int code) {
+  if (me::umma::mbar_wait(bar, parity, rules.tries, stop)) return true;
+  if (!*stop) atomicCAS(err, 0, code);
+  *stop = 1;
+  return false;
+}
 
 // values k and k + 1 (k even, so both or neither are in) of a profile
 template <bool VEC>
@@ -778,24 +799,26 @@ __global__ void __launch_bounds__(kPredThreads, 1)
                        const __grid_constant__ CUtensorMap w1,
                        const __grid_constant__ CUtensorMap w2,
                        const __grid_constant__ CUtensorMap w3, const PredNet net,
+                       const __grid_constant__ WaitRules rules,
                        const double *__restrict__ prof, long long n, int nl, int nip,
                        double *__restrict__ par, int *__restrict__ err) {
   using namespace me::umma;
   extern __shared__ __align__(1024) uint8_t pred_smem[];
   const uint32_t base = smem_u32(pred_smem);
   const uint32_t sW = base + 2 * kPredA, bars = sW + kPredStages * kPredStage;
-  // full[s] = bars + 8 s, empty[s] after them, then done[tile]
-  const uint32_t done = bars + 8 * 2 * kPredStages;
-  uint32_t *misc = reinterpret_cast<uint32_t *>(pred_smem + (done + 16 - base));
-  volatile uint32_t *abort_flag = misc + 1;
+  // full[s] = bars + 8 s, empty[s] after them, then done[tile], drain, and one for
+  // each stage and tile that nothing waits for
+  const uint32_t done = bars + 8 * 2 * kPredStages, drain = done + 16, spare = drain + 8;
+  uint32_t *misc = reinterpret_cast<uint32_t *>(pred_smem + (spare + 8 * kPredStages - base));
+  volatile uint32_t *stop = misc + 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp == 0) {
     tmem_alloc(smem_u32(misc), 512);
     tmem_relinquish();
   }
   if (threadIdx.x == 32) {
-    for (int s = 0; s < 2 * kPredStages + 2; s++) mbar_init(bars + 8 * s, 1);
-    *abort_flag = (base & 1023u) ? 1u : 0u;
+    for (int s = 0; s < 3 * kPredStages + 3; s++) mbar_init(bars + 8 * s, 1);
+    *stop = (base & 1023u) ? 1u : 0u;
     if (base & 1023u) atomicExch(err, 1);  // the tiles need their alignment
     mbar_fence_init();
   }
@@ -814,8 +837,9 @@ __global__ void __launch_bounds__(kPredThreads, 1)
   const int phases = pieces + 3;
   auto blocks_of = [&](int ph) { return ph == pieces - 1 ? last_blocks : 4; };
   if (warp == 2 * kPredWarps + 1) {
-    if (lane == 0 && !*abort_flag) {
+    if (lane == 0 && !*stop) {
       uint32_t st = 0, par = 1;  // parity that empty[st] waits for (fresh: passes)
+      const uint32_t landed = rules.drop == 1 ? spare : bars;
       bool dead = false;
       for (int todo = (int)mine0; todo > 0 && !dead; todo -= 2) {
         if (VEC)  // the next pair's profiles into L2
@@ -827,11 +851,11 @@ __global__ void __launch_bounds__(kPredThreads, 1)
         for (int ph = 0; ph < phases && !dead; ph++)
           for (int g = 0; g < 2 && g < todo && !dead; g++)
             for (int kb = 0; kb < blocks_of(ph); kb++) {
-              if (!mbar_wait(bars + 8 * (kPredStages + st), par)) {
-                dead = true;  // (or the MMAs have stopped)
+              if (!role_wait(bars + 8 * (kPredStages + st), par, rules, stop, err, 2)) {
+                dead = true;
                 break;
               }
-              const uint32_t full = bars + 8 * st, dst = sW + st * kPredStage;
+              const uint32_t full = landed + 8 * st, dst = sW + st * kPredStage;
               if (ph == phases - 1) {
                 mbar_expect_tx(full, 32 * kBK * 2);
                 tma_load_2d(dst, &w3, full, kb * kBK, 0);
@@ -845,18 +869,16 @@ __global__ void __launch_bounds__(kPredThreads, 1)
               if (++st == kPredStages) st = 0, par ^= 1;
             }
       }
-      if (dead) {
-        *abort_flag = 1;
-        atomicExch(err, 2);
-        // copies that no MMA will read: let them land
-        for (uint32_t i = 0; i < kPredStages; i++)
-          mbar_wait(bars + 8 * i, i < st ? par ^ 1 : par);
-      }
+      // the last copies, which no MMA may have read, land before the CTA ends
+      for (uint32_t i = 0; i < kPredStages; i++)
+        mbar_wait(landed + 8 * i, i < st ? par ^ 1 : par, rules.tries);
     }
     __syncwarp();
   } else if (warp == 2 * kPredWarps) {
     uint32_t st = 0, par = 0;
-    bool dead = *abort_flag != 0;
+    const uint32_t freed = rules.drop == 3 ? spare : bars + 8 * kPredStages;
+    const uint32_t ended = rules.drop == 2 ? spare : done;
+    bool dead = *stop != 0;
     const uint64_t descW = sw128_kmajor_desc(sW);
     for (int todo = (int)mine0; todo > 0; todo -= 2)
       for (int ph = 0; ph < phases; ph++)
@@ -866,16 +888,15 @@ __global__ void __launch_bounds__(kPredThreads, 1)
           else
             asm volatile("bar.sync 2, %0;" ::"n"((kPredWarps + 1) * 32) : "memory");
           tc_fence_after();
-          if (lane == 0) {
+          if (lane == 0 && !dead) {
             const uint32_t idesc = idesc_bf16_f32(kBM, ph == phases - 1 ? 32 : 256);
             uint64_t da = sw128_kmajor_desc(base + g * kPredA);
             const uint32_t d = tmem + (uint32_t)(g * 256);
             const int count = blocks_of(ph);
             const bool fresh = ph == 0 || ph >= pieces;
-            for (int kb = 0; kb < count && !dead; kb++) {
-              if (!mbar_wait(bars + 8 * st, par)) {
+            for (int kb = 0; kb < count; kb++) {
+              if (!role_wait(bars + 8 * st, par, rules, stop, err, 1)) {
                 dead = true;
-                atomicExch(err, 1);
                 break;
               }
               tc_fence_after();
@@ -885,19 +906,19 @@ __global__ void __launch_bounds__(kPredThreads, 1)
               umma_bf16(d, da + 2, db + 2, idesc, 1);
               umma_bf16(d, da + 4, db + 4, idesc, 1);
               umma_bf16(d, da + 6, db + 6, idesc, 1);
-              mma_commit(bars + 8 * (kPredStages + st));
+              mma_commit(freed + 8 * st);
               da += kStageA >> 4;
               if (++st == kPredStages) st = 0, par ^= 1;
             }
-            if (dead) {
-              *abort_flag = 1;
-              mbar_arrive(done + 8 * g);
-            } else {
-              mma_commit(done + 8 * g);
-            }
+            if (!dead) mma_commit(ended + 8 * g);
           }
           __syncwarp();
         }
+    if (lane == 0 && *stop) {  // what it issued ends before the CTA does
+      mma_commit(drain);
+      mbar_wait(drain, 0, rules.tries);
+    }
+    __syncwarp();
   } else {
     const int g = warp / kPredWarps, gw = warp % kPredWarps;
     uint8_t *tileA = pred_smem + g * kPredA;
@@ -907,9 +928,9 @@ __global__ void __launch_bounds__(kPredThreads, 1)
       fence_smem_to_async();
       tc_fence_before();
       if (g == 0)
-        asm volatile("bar.arrive 1, %0;" ::"n"((kPredWarps + 1) * 32) : "memory");
+        asm volatile("bar.sync 1, %0;" ::"n"((kPredWarps + 1) * 32) : "memory");
       else
-        asm volatile("bar.arrive 2, %0;" ::"n"((kPredWarps + 1) * 32) : "memory");
+        asm volatile("bar.sync 2, %0;" ::"n"((kPredWarps + 1) * 32) : "memory");
     };
     auto group_sync = [&]() {
       if (g == 0)
@@ -918,10 +939,8 @@ __global__ void __launch_bounds__(kPredThreads, 1)
         asm volatile("bar.sync 4, %0;" ::"n"(kPredWarps * 32) : "memory");
     };
     auto finished = [&]() {  // this phase's MMAs are done
-      if (!mbar_wait(done + 8 * g, phase & 1u)) {
-        *abort_flag = 1;
-        atomicExch(err, 3);
-      }
+      role_wait(done + 8 * g, phase & 1u, rules, stop, err, 3);
+      __syncwarp();
       phase++;
       tc_fence_after();
     };
@@ -1031,7 +1050,7 @@ __global__ void __launch_bounds__(kPredThreads, 1)
         const long long i = tile * kBM + row;
 #pragma unroll
         for (int j = 0; j < kOut; j++) y[j] += __ldg(net.bias[3] + j);
-        if (i < n && !*abort_flag)
+        if (i < n && !*stop)
           decode_row(y, net.tmean, net.tstd, s_imax[row], par + (size_t)i * 9);
       }
       group_sync();  // the next tile's I_max must not overtake the decode
@@ -1096,26 +1115,27 @@ __device__ __forceinline__ uint32_t step_offset(int row, int k) {
 
 __global__ void __launch_bounds__(kStepThreads, 1)
     mlp_step_kernel(const __grid_constant__ StepMaps maps, const __grid_constant__ StepNet net,
-                    const bf16 *__restrict__ X, const long long *__restrict__ idx,
-                    const float *__restrict__ T, int B, int nip, double *__restrict__ loss,
-                    int *__restrict__ err) {
+                    const __grid_constant__ WaitRules rules, const bf16 *__restrict__ X,
+                    const long long *__restrict__ idx, const float *__restrict__ T, int B,
+                    int nip, double *__restrict__ loss, int *__restrict__ err) {
   using namespace me::umma;
   extern __shared__ __align__(1024) uint8_t step_smem[];
   const uint32_t base = smem_u32(step_smem);
   uint8_t *tile = step_smem + kStepStages * kPredStage;
   const uint32_t sX = base + kStepStages * kPredStage, bars = sX + 4 * kStepBlock;
-  // full[s] = bars + 8 s, empty[s] after them, then done
-  const uint32_t done = bars + 8 * 2 * kStepStages;
-  uint32_t *misc = reinterpret_cast<uint32_t *>(step_smem + (done + 8 - base));
-  volatile uint32_t *abort_flag = misc + 1;
+  // full[s] = bars + 8 s, empty[s] after them, then done, drain and the spare
+  // ones; waits and barriers as in mlp_predict_kernel
+  const uint32_t done = bars + 8 * 2 * kStepStages, drain = done + 8, spare = drain + 8;
+  uint32_t *misc = reinterpret_cast<uint32_t *>(step_smem + (spare + 8 * kStepStages - base));
+  volatile uint32_t *stop = misc + 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp == 0) {
     tmem_alloc(smem_u32(misc), 64);
     tmem_relinquish();
   }
   if (threadIdx.x == 32) {
-    for (int s = 0; s < 2 * kStepStages + 1; s++) mbar_init(bars + 8 * s, 1);
-    *abort_flag = (base & 1023u) ? 1u : 0u;
+    for (int s = 0; s < 3 * kStepStages + 2; s++) mbar_init(bars + 8 * s, 1);
+    *stop = (base & 1023u) ? 1u : 0u;
     if (base & 1023u) atomicExch(err, 1);  // the tiles need their alignment
     mbar_fence_init();
   }
@@ -1132,19 +1152,20 @@ __global__ void __launch_bounds__(kStepThreads, 1)
   auto blocks_of = [&](int ph) { return ph == pieces - 1 ? last_blocks : ph == out + 1 ? 1 : 4; };
 
   if (warp == kStepWarps + 1) {
-    if (lane == 0 && !*abort_flag) {
+    if (lane == 0 && !*stop) {
       uint32_t st = 0, par = 1;  // parity that empty[st] waits for (fresh: passes)
+      const uint32_t landed = rules.drop == 1 ? spare : bars;
       bool dead = false;
       for (int ph = 0; ph < phases && !dead; ph++) {
         const CUtensorMap *w = ph < pieces ? &maps.w[0]
                                : ph <= out ? &maps.w[ph - pieces + 1]
                                            : &maps.t[kLayers - (ph - out)];
         for (int kb = 0; kb < blocks_of(ph); kb++) {
-          if (!mbar_wait(bars + 8 * (kStepStages + st), par)) {
-            dead = true;  // (or the MMAs have stopped)
+          if (!role_wait(bars + 8 * (kStepStages + st), par, rules, stop, err, 2)) {
+            dead = true;
             break;
           }
-          const uint32_t full = bars + 8 * st, dst = base + st * kPredStage;
+          const uint32_t full = landed + 8 * st, dst = base + st * kPredStage;
           const int k = (ph < pieces ? ph * kPredK : 0) + kb * kBK;
           mbar_expect_tx(full, ph == out ? 32 * kBK * 2 : kPredStage);
           tma_load_2d(dst, w, full, k, 0);
@@ -1152,31 +1173,28 @@ __global__ void __launch_bounds__(kStepThreads, 1)
           if (++st == kStepStages) st = 0, par ^= 1;
         }
       }
-      if (dead) {
-        *abort_flag = 1;
-        atomicExch(err, 2);
-        // copies that no MMA will read: let them land
-        for (uint32_t i = 0; i < kStepStages; i++)
-          mbar_wait(bars + 8 * i, i < st ? par ^ 1 : par);
-      }
+      // the last copies, which no MMA may have read, land before the CTA ends
+      for (uint32_t i = 0; i < kStepStages; i++)
+        mbar_wait(landed + 8 * i, i < st ? par ^ 1 : par, rules.tries);
     }
     __syncwarp();
   } else if (warp == kStepWarps) {
     uint32_t st = 0, par = 0;
-    bool dead = *abort_flag != 0;
+    const uint32_t freed = rules.drop == 3 ? spare : bars + 8 * kStepStages;
+    const uint32_t ended = rules.drop == 2 ? spare : done;
+    bool dead = *stop != 0;
     const uint64_t descW = sw128_kmajor_desc(base);
     const uint32_t idesc = idesc_bf16_f32(kBM, kStepRows);
     for (int ph = 0; ph < phases; ph++) {
       asm volatile("bar.sync 1, %0;" ::"n"((kStepWarps + 1) * 32) : "memory");
       tc_fence_after();
-      if (lane == 0) {
+      if (lane == 0 && !dead) {
         uint64_t db = sw128_kmajor_desc(sX);
         const int count = blocks_of(ph);
         const bool fresh = ph == 0 || ph >= pieces;
-        for (int kb = 0; kb < count && !dead; kb++) {
-          if (!mbar_wait(bars + 8 * st, par)) {
+        for (int kb = 0; kb < count; kb++) {
+          if (!role_wait(bars + 8 * st, par, rules, stop, err, 1)) {
             dead = true;
-            atomicExch(err, 1);
             break;
           }
           tc_fence_after();
@@ -1189,34 +1207,32 @@ __global__ void __launch_bounds__(kStepThreads, 1)
             if (ph != out)
               umma_bf16(tmem + kStepRows, da + (kPredBox >> 4) + 2 * k, db + 2 * k, idesc, add);
           }
-          mma_commit(bars + 8 * (kStepStages + st));
+          mma_commit(freed + 8 * st);
           db += kStepBlock >> 4;
           if (++st == kStepStages) st = 0, par ^= 1;
         }
-        if (dead) {
-          *abort_flag = 1;
-          mbar_arrive(done);
-        } else {
-          mma_commit(done);
-        }
+        if (!dead) mma_commit(ended);
       }
       __syncwarp();
     }
+    if (lane == 0 && *stop) {  // what it issued ends before the CTA does
+      mma_commit(drain);
+      mbar_wait(drain, 0, rules.tries);
+    }
+    __syncwarp();
   } else {
     uint32_t phase = 0;
     auto publish = [&]() {  // the operand is written and the accumulator read
       fence_smem_to_async();
       tc_fence_before();
-      asm volatile("bar.arrive 1, %0;" ::"n"((kStepWarps + 1) * 32) : "memory");
+      asm volatile("bar.sync 1, %0;" ::"n"((kStepWarps + 1) * 32) : "memory");
     };
     auto workers = [&]() {
       asm volatile("bar.sync 2, %0;" ::"n"(kStepWarps * 32) : "memory");
     };
     auto finished = [&]() {  // this phase's MMAs are done
-      if (!mbar_wait(done, phase & 1u)) {
-        *abort_flag = 1;
-        atomicExch(err, 3);
-      }
+      role_wait(done, phase & 1u, rules, stop, err, 3);
+      __syncwarp();
       phase++;
       tc_fence_after();
     };
@@ -1602,6 +1618,7 @@ struct me_mlp {
   // moments and their gradients have one layout, of `flat` floats each
   DBuf model, batch, step;
   long long flat = 0;
+  WaitRules waits;  // of the fused kernels (me_mlp_set_waits)
   // GEMM kernel choice and the tcgen05 kernel's error flag (device int)
   GemmPath gemm_path = GemmPath::tcgen05;
   DBuf gerr;
@@ -1901,7 +1918,7 @@ void plan_step(me_mlp *m, int B, StepPlan *p) {
 void run_step(me_mlp *m, const StepPlan &p, int B, const bf16 *X, const float *T,
               const long long *idx, cudaStream_t st) {
   mlp_step_kernel<<<B / kStepRows, kStepThreads, kStepSmem, st>>>(
-      p.maps, p.net, X, idx, T, B, m->nip, m->loss.as<double>(), m->gerr.as<int>());
+      p.maps, p.net, m->waits, X, idx, T, B, m->nip, m->loss.as<double>(), m->gerr.as<int>());
   mlp_wgrad_kernel<<<dim3(p.tiles, p.split), 128, me::umma::smem_bytes(kGradN), st>>>(
       p.gmaps, p.gnet, B, m->gerr.as<int>());
   m->gemm_launches[(int)GemmPath::tcgen05] += kLayers + 2 * kLayers - 1;
@@ -2156,8 +2173,8 @@ static bool predict_fused(me_mlp *m, const double *d_prof, long npix, double *d_
   const long long tiles = ((long long)npix + me::umma::kBM - 1) / me::umma::kBM;
   const unsigned grid = (unsigned)(tiles < dv.sms ? tiles : dv.sms);
   auto go = [&](auto kernel) {
-    kernel<<<grid, kPredThreads, kPredSmem, st>>>(w[0], w[1], w[2], w[3], net, d_prof, npix, m->nl,
-                                                  m->nip, d_par, m->gerr.as<int>());
+    kernel<<<grid, kPredThreads, kPredSmem, st>>>(w[0], w[1], w[2], w[3], net, m->waits, d_prof,
+                                                  npix, m->nl, m->nip, d_par, m->gerr.as<int>());
   };
   if ((reinterpret_cast<uintptr_t>(d_prof) & 15) == 0)
     go(mlp_predict_kernel<true>);
@@ -2305,6 +2322,15 @@ extern "C" int me_mlp_set_gemm(me_mlp *m, int path) {
   if (path != ME_GEMM_TCGEN05 && path != ME_GEMM_MMA_SYNC)
     return fail(ME_ERR_ARG, "path must be ME_GEMM_TCGEN05 or ME_GEMM_MMA_SYNC");
   m->gemm_path = path == ME_GEMM_TCGEN05 ? GemmPath::tcgen05 : GemmPath::mma_sync;
+  return ME_OK;
+}
+
+extern "C" int me_mlp_set_waits(me_mlp *m, unsigned tries, int drop) {
+  if (!m) return fail(ME_ERR_ARG, "null argument");
+  if (drop < 0 || drop > 3) return fail(ME_ERR_ARG, "drop must be 0 to 3");
+  m->waits = WaitRules();
+  if (tries) m->waits.tries = tries;
+  m->waits.drop = drop;
   return ME_OK;
 }
 

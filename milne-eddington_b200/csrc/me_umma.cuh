@@ -43,8 +43,10 @@ __host__ __device__ constexpr int smem_bytes(int bn) {
              : (kSmPerSm / (512 / (int)tmem_cols(bn) + 1) - kSmPerCta + 1);
 }
 constexpr int kSmemMax = smem_bytes(kMaxBN);
-// give up a wait after 2 s of device time (or 2^26 polls)
-constexpr unsigned long long kWaitNs = 2000000000ull;
+// Waits give up after so many tries of mbarrier.try_wait (140 to 290 ns each on a
+// B200: some 2 s).  Tries, not time: a GPU that was taken away from the kernel for
+// a while does not end its waits.
+constexpr uint32_t kWaitTries = 1u << 23;
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return (uint32_t)__cvta_generic_to_shared(p);
@@ -75,24 +77,15 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
-__device__ __forceinline__ unsigned long long now_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
 // Waits for the completion of the phase of parity `parity`; false when it has
-// not completed within kWaitNs (the caller records an error and stops).
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-  // (the timer is read only once the first tries have failed)
-  unsigned long long t0 = 0;
-  for (uint32_t it = 1; it < (1u << 26); it++) {
+// not completed within so many tries (the caller records an error and stops), or
+// when *stop is found raised (another warp of the CTA has given up).
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity,
+                                          uint32_t tries = kWaitTries,
+                                          const volatile uint32_t *stop = nullptr) {
+  for (uint32_t it = tries; it; it--) {
     if (mbar_try(bar, parity)) return true;
-    if ((it & 63) == 0) {
-      const unsigned long long t = now_ns();
-      if (!t0) t0 = t;
-      if (t - t0 > kWaitNs) return false;
-    }
+    if ((it & 63) == 0 && stop && *stop) return false;
   }
   return false;
 }

@@ -152,7 +152,7 @@ EXPORTED = [
     "me_mlp_shape", "me_mlp_get_params", "me_mlp_set_params", "me_mlp_loss_grad",
     "me_fits_image_info", "me_fits_read", "me_fits_create", "me_fits_write",
     "me_run_options_default", "me_run", "me_run_config", "me_plan_set_filter",
-    "me_mlp_set_gemm", "me_mlp_gemm_launches", "me_gemm_bf16", "me_plan_set_queue_order",
+    "me_mlp_set_gemm", "me_mlp_set_waits", "me_mlp_gemm_launches", "me_gemm_bf16", "me_plan_set_queue_order",
     "me_order_by_key", "me_plan_poll_trace", "me_plan_set_drain", "me_plan_get_drain",
     "me_plan_faddeeva", "me_plan_set_faddeeva", "me_plan_givens", "me_plan_set_givens",
     "me_plan_set_slot_profiles", "me_weideman16", "me_faddeeva_weideman",
@@ -360,6 +360,7 @@ def lib() -> ctypes.CDLL:
         L.me_mlp_set_params.argtypes = [ctypes.c_void_p, _F]
         L.me_mlp_loss_grad.argtypes = [ctypes.c_void_p, _F, _F, ctypes.c_int, _D, _F]
         L.me_mlp_set_gemm.argtypes = [ctypes.c_void_p, ctypes.c_int]
+        L.me_mlp_set_waits.argtypes = [ctypes.c_void_p, ctypes.c_uint, ctypes.c_int]
         L.me_mlp_gemm_launches.argtypes = [ctypes.c_void_p, ctypes.POINTER(ctypes.c_longlong),
                                            ctypes.POINTER(ctypes.c_longlong)]
         _U16 = ctypes.POINTER(ctypes.c_uint16)
@@ -886,6 +887,11 @@ class Initializer:
         """"tcgen05" (the default) or "mma_sync": the GEMM kernel of training and
         inference."""
         _check(lib().me_mlp_set_gemm(self._h, GEMM_PATHS[path]), "me_mlp_set_gemm")
+
+    def set_waits(self, tries: int = 0, drop: int = 0):
+        """For tests: the limit of the fused kernels' waits (0: the default), and events that
+        go unannounced (1 loads of weights, 2 MMAs' completion, 3 stages' release)."""
+        _check(lib().me_mlp_set_waits(self._h, tries, drop), "me_mlp_set_waits")
 
     def gemm_launches(self):
         """{"tcgen05": n, "mma_sync": n}: GEMM launches of each kernel so far."""
