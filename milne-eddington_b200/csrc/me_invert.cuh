@@ -1726,9 +1726,12 @@ __global__ void __launch_bounds__(TailShape<T, FILT>::kThreads, 1)
     while (true) {
       tail_sync<Sh::kSynth>();
       const int st = sm.slot.state;
-      if (st == SL_DONE || st == SL_EMPTY || sm.ctl.error) break;
+      const bool over = st == SL_DONE || st == SL_EMPTY || sm.ctl.error;
+      // every thread has read them before thread 0 moves on (a run that ends
+      // without a trial has no other barrier on its way to the transition)
+      tail_sync<Sh::kSynth>();
+      if (over) break;
       if (++steps > cap) {  // cannot happen for a valid plan
-        tail_sync<Sh::kSynth>();
         if (tid == 0) sm.ctl.error = 1;
         continue;
       }
