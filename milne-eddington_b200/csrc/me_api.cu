@@ -1575,7 +1575,11 @@ extern "C" int me_plan_autotune(me_plan *p, const double *d_prof, long npix, voi
       {&p->tail_slots,
        {0, p->sms * me::kTailPerSm / 2, -1, p->sms * me::kTailPerSm * 2,
         p->sms * me::kTailPerSm * 4}},
-      {&p->svd_lanes, {1, 2}},
+      // lanes per matrix in the full rounds; with all nine parameters free the
+      // solves run one thread per matrix whatever it says, and it would only
+      // change their rounding
+      {&p->svd_lanes,
+       p->P.npar < 9 ? std::vector<int>{1, 2} : std::vector<int>{p->svd_lanes}},
       // the Jacobian / trial kernels' variant: 64, 128 or 256 pixels per CTA,
       // the wavelength grid staged in shared memory, no reciprocal table, the
       // normal-equation sums in shared memory
