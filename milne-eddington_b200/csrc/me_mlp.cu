@@ -743,8 +743,8 @@ __global__ void decode_kernel(const float *Y, long long n, int ld, const float *
 // decode_kernel, which did this in six launches with every layer's activations
 // through memory.  Profiles of 60 wavelengths, there and here, us:
 //   1: 46, 45;  1,000: 53, 47;  18,900: 90, 50;  37,889: 162, 95;  300,007: 921, 493
-// and of 112: 1: 52, 51;  18,900: 106, 56;  75,000: 313, 163.  So it is used at
-// every count; the six launches remain for the mma.sync GEMMs.
+// and of 112: 1: 52, 51;  18,900: 106, 56;  75,000: 313, 163.  Few profiles of
+// more features go through the six launches all the same: see predict_separately.
 // Waits are bounded.  The first to run out writes a code to *err (1: weights, 2: a
 // free stage, 3: the accumulator) and raises the CTA's stop flag, at which all
 // other waits end too.  The named barriers have no limit: every warp passes each
@@ -1612,6 +1612,7 @@ struct me_mlp {
   // batch work buffers
   int cap = 0, step_cap = 0;
   DBuf xb, xbt, z[kLayers], a[kLayers], at[kLayers], yf, dyb, dybt, dh, dz, dzt;
+  cudaEvent_t batch_used = nullptr;  // the last inference that used them
   DBuf sxt, sat[kLayers - 1], sdzt[kLayers];  // operands of the weight gradients (mlp_step_kernel)
   DBuf loss, imax;
   // the allocations that the buffers above are parts of; the parameters, their
@@ -1624,6 +1625,9 @@ struct me_mlp {
   DBuf gerr;
   long long gemm_launches[2] = {0, 0};
   TileMapCache maps;
+  ~me_mlp() {
+    if (batch_used) cudaEventDestroy(batch_used);
+  }
 };
 
 namespace {
@@ -1958,6 +1962,17 @@ void prior_from(const me_mlp_train_params *tp, Prior &pr) {
   pr.meta_hi = (float)tp->mix_eta_range[1];
 }
 
+// Few profiles of many features: the separate kernels, whose features kernel has a
+// warp per profile and a CTA per eight, where mlp_predict_kernel's CTA of 128
+// takes them piece by piece.  Both sides, us for a call alone, separately and in
+// one kernel: 1 profile of 112 wavelengths 47.8, 49.6; 128: 45.2, 50.4; 192: 49.0,
+// 54.5; 512: 63.4, 84.8; 64 of 128: 48.3, 51.4; 128 of 128: 53.5, 52.8, and of 160:
+// 55.1, 55.0; 3,000 of 193: 62.8, 63.3, and of 512: 88.7, 95.1; 5,000 of 256: 75.5,
+// 67.8, and of 512: 106.9, 97.3.  The values are the same.
+bool predict_separately(const me_mlp *m, long long npix) {
+  return m->nip > 384 && npix <= (m->nip > 768 ? 3072 : 64);
+}
+
 }  // namespace
 
 namespace me {
@@ -1967,7 +1982,8 @@ int plan_devplan(const me_plan *p, DevPlan *out, int *device);
 int mlp_gemm_status(me_mlp *m) { return gemm_status(m); }
 
 long long mlp_predict_launches(const me_mlp *m, long long npix) {
-  return m->gemm_path == GemmPath::tcgen05 && device_facts().pred_ok
+  return m->gemm_path == GemmPath::tcgen05 && device_facts().pred_ok &&
+                 !predict_separately(m, npix)
              ? 1
              : kMlpPredLaunches * ((npix + kMlpPredChunk - 1) / kMlpPredChunk);
 }
@@ -2191,7 +2207,13 @@ extern "C" int me_mlp_predict_device(me_mlp *m, const double *d_prof, long npix,
   if (npix == 0) return ME_OK;
   MCK(cudaSetDevice(m->device));
   cudaStream_t st = (cudaStream_t)stream;
-  if (predict_fused(m, d_prof, npix, d_par, st)) {
+  // (the separate kernels share the initialiser's buffers, which a first call
+  // allocates: not under capture, and in order from stream to stream)
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  const bool apart = predict_separately(m, npix) &&
+                     cudaStreamIsCapturing(st, &capture) == cudaSuccess &&
+                     capture == cudaStreamCaptureStatusNone;
+  if (!apart && predict_fused(m, d_prof, npix, d_par, st)) {
     MCK(cudaGetLastError());
     if (!stream) {
       MCK(cudaStreamSynchronize(st));
@@ -2202,6 +2224,10 @@ extern "C" int me_mlp_predict_device(me_mlp *m, const double *d_prof, long npix,
   const int chunk = (int)(npix < me::kMlpPredChunk ? (npix + 255) / 256 * 256 : me::kMlpPredChunk);
   int rc = ensure_batch(m, chunk);
   if (rc) return rc;
+  if (apart) {
+    if (!m->batch_used) MCK(cudaEventCreateWithFlags(&m->batch_used, cudaEventDisableTiming));
+    MCK(cudaStreamWaitEvent(st, m->batch_used, 0));
+  }
   for (long long r0 = 0; r0 < npix; r0 += chunk) {
     const int rows = (int)((npix - r0) < chunk ? (npix - r0) : chunk);
     // a chunk starts 32 nl r0 bytes in, so its alignment is the base's
@@ -2219,6 +2245,7 @@ extern "C" int me_mlp_predict_device(me_mlp *m, const double *d_prof, long npix,
                                                    m->imax.as<float>(), d_par + (size_t)r0 * 9);
   }
   MCK(cudaGetLastError());
+  if (apart) MCK(cudaEventRecord(m->batch_used, st));
   if (!stream) {
     MCK(cudaStreamSynchronize(st));
     return gemm_status(m);
@@ -2287,6 +2314,7 @@ extern "C" int me_mlp_loss_grad(me_mlp *m, const float *x, const float *t, int r
   MCK(cudaSetDevice(m->device));
   int rc = ensure_batch(m, rows);
   if (rc) return rc;
+  if (m->batch_used) MCK(cudaStreamWaitEvent(nullptr, m->batch_used, 0));
   DBuf xf, tf, idx;
   MCK(xf.ensure((size_t)rows * m->nip * 4));
   MCK(tf.ensure((size_t)rows * kOut * 4));
