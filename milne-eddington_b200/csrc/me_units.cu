@@ -411,6 +411,15 @@ cudaError_t launch_round(int precision, const DevPlan &P, const InvertArgs &A, c
   return ME_PICK(launch_round, P, A, S, parity, grids, st, ev, svd_lanes, ov);
 }
 
+// SMs of the current device
+static long long device_sms() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return 1;
+  return sms > 0 ? sms : 1;
+}
+
 template <class T>
 static void launch_synth_t(const DevPlan &P, const double *d_par, const unsigned char *d_flags,
                            long long npix, double step7, double *d_prof, double *d_jac,
@@ -419,15 +428,16 @@ static void launch_synth_t(const DevPlan &P, const double *d_par, const unsigned
   // four blocks per SM, so that a few pixels spread over the device; of the
   // upper half of that range, the count whose wavelengths leave the fewest of
   // the block's threads idle in its last pass (6 wavelengths: 21 pixels)
-  constexpr long long kBlocks = 148 * 4;
-  int per = kSynthPixels<T>;
-  while (per > 1 && (npix + per - 1) / per < kBlocks) per /= 2;
+  const long long sms = device_sms();
+  constexpr int kMost = kSynthPixels<T>;
+  int per = kMost;
+  while (per > 1 && (npix + per - 1) / per < sms * 4) per /= 2;
   auto used = [&](int n) {
     const int points = n * P.nl;
     return (double)points / ((points + kSynthThreads - 1) / kSynthThreads * kSynthThreads);
   };
-  if (per == kSynthPixels<T>)
-    for (int n = per - 1; n >= per / 2; n--)
+  if (per == kMost)
+    for (int n = kMost - 1; n >= kMost / 2; n--)
       if (used(n) > used(per) + 0.05) per = n;
   const unsigned g = (unsigned)((npix + per - 1) / per);
   // with a filter a point is a sub-wavelength, its terms staged in shared
@@ -437,7 +447,7 @@ static void launch_synth_t(const DevPlan &P, const double *d_par, const unsigned
   // against 18).  FP64 Jacobians are always split: 40 sums of doubles beside
   // the point's registers spill (17486 pixels 1231 us against 906)
   const int mode = P.nsub <= 1 ? kPlain
-                   : npix * P.nl >= 148 * (d_jac ? 512 : 1024) ? kFilter : kFilterSplit;
+                   : npix * P.nl >= sms * (d_jac ? 512 : 1024) ? kFilter : kFilterSplit;
   auto go = [&](auto jac, auto m) {
     synth_kernel<T, jac.value, m.value><<<g, kSynthThreads, 0, st>>>(
         P, d_par, d_flags, npix, per, step7, d_prof, d_jac);
@@ -495,8 +505,9 @@ cudaError_t launch_voigt(int precision, const DevPlan &P, const double *d_nu, co
 // which eight warps per SM cover them at once; a warp's time is that of the
 // longest of its matrices' sweeps
 static int svd_per_warp(long long nmat) {
+  const long long warps = device_sms() * 8;
   int per = 32;
-  while (per > 1 && (nmat + per / 2 - 1) / (per / 2) <= 148 * 8) per /= 2;
+  while (per > 1 && (nmat + per / 2 - 1) / (per / 2) <= warps) per /= 2;
   return per;
 }
 
