@@ -273,6 +273,12 @@ __device__ __noinline__ HL<T> voigt_humlicek_w4(T nu, T y) {
   return {H, L};
 }
 
+// The first term of Alg 916's series, in a range where the terms after it can be
+// counted: x + y <= 1e7 keeps it there by itself, but a NaN among them passes
+// every test of the regions, and converts to the least integer, or leaves an x
+// of any size.  (The counts of terms are cut off at 0 for the same reason.)
+__device__ __forceinline__ int term_index(int nb) { return min(max(nb, 0), 1 << 30); }
+
 // FP32 form of Alg 916 with the same series, terms and cut-offs, arranged for
 // the GPU: the 1 / (a^2 n^2 + y^2) factors come from the per-synthesis table;
 // with d_b = x - a n_b and d_f = a - d_b (n_f = n_b + 1), exp(-d_f^2) and
@@ -305,12 +311,12 @@ __device__ __forceinline__ HL<float> voigt_alg916_f32(float nu, float y, float e
   const int nmax2 = (int)((K.sqrt_log_rmin0 - x) * K.inv_a + 0.5f);
   int nmax = nmax1 > nmax2 ? nmax1 : nmax2;
   if (nmax >= K.nmax) nmax = K.nmax - 1;
-  const int nb = (int)(x * K.inv_a + 0.5f);
+  const int nb = term_index((int)(x * K.inv_a + 0.5f));
   const int nf = nb + 1;
   const float dxb = x - a * nb;
   const float dxf = a - dxb;
-  int nmaxf = (int)((K.sqrt_log_rmin0 - dxf) * K.inv_a);
-  int nmaxb = (int)((K.sqrt_log_rmin0 - dxb) * K.inv_a);
+  int nmaxf = max((int)((K.sqrt_log_rmin0 - dxf) * K.inv_a), 0);
+  int nmaxb = max((int)((K.sqrt_log_rmin0 - dxb) * K.inv_a), 0);
   if (nmaxf >= K.nmax) nmaxf = K.nmax - 1;
   if (nmaxb >= K.nmax) nmaxb = K.nmax - 1;
   const int nlo = (nb - nmaxb) > 1 ? (nb - nmaxb) : 1;
@@ -393,12 +399,12 @@ __device__ __forceinline__ HL<T> voigt_alg916(T nu, T y, T erfcx_y, const VoigtK
   const int nmax2 = (int)((K.sqrt_log_rmin0 - x) / a + T(0.5));
   int nmax = nmax1 > nmax2 ? nmax1 : nmax2;
   if (nmax >= K.nmax) nmax = K.nmax - 1;
-  const int nb = (int)(x / a + T(0.5));
+  const int nb = term_index((int)(x / a + T(0.5)));
   const int nf = nb + 1;
   const T dxf = a * nf - x;
   const T dxb = x - a * nb;
-  int nmaxf = (int)((K.sqrt_log_rmin0 - dxf) / a);
-  int nmaxb = (int)((K.sqrt_log_rmin0 - dxb) / a);
+  int nmaxf = max((int)((K.sqrt_log_rmin0 - dxf) / a), 0);
+  int nmaxb = max((int)((K.sqrt_log_rmin0 - dxb) / a), 0);
   if (nmaxf >= K.nmax) nmaxf = K.nmax - 1;
   if (nmaxb >= K.nmax) nmaxb = K.nmax - 1;
   const int nlo = (nb - nmaxb) > 1 ? (nb - nmaxb) : 1;
