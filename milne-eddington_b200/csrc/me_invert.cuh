@@ -434,9 +434,12 @@ __device__ __forceinline__ void jac_store(const DevPlan &P, const Slots &S, int 
 // and rv1 likewise.  G > 1: a group of G lanes (`mask`), the matrix
 // row-major in the group's shared memory, w and rv1 private to each lane (the
 // decomposition is gr_svd_u_grp, the rest runs redundantly in every lane and
-// lane 0 stores).  Returns the number of decompositions that hit the 50-sweep
-// limit.
-template <int STR, int G>
+// lane 0 stores).  NINE: the caller may have all nine parameters free, whose
+// decomposition by a warp has a form of its own (in a kernel that never has, its
+// registers would only cost residency: svd_grp_kernel<32> 96 with it left out,
+// 255 with it, and 15 % of its time).  Returns the number of decompositions that
+// hit the 50-sweep limit.
+template <int STR, int G, bool NINE = false>
 __device__ __forceinline__ int solve_slot(const DevPlan &P, const Slots &S, int s, double *a,
                                           double *w, double *rv1, int lane, unsigned mask) {
   constexpr bool WARP = G > 1;
@@ -450,7 +453,7 @@ __device__ __forceinline__ int solve_slot(const DevPlan &P, const Slots &S, int 
   for (int k = WARP ? lane : 0; k < n * n; k += G) a[k * STR] = S.hess[(size_t)k * W + s];
   if (WARP) __syncwarp(mask);
   auto decompose = [&]() {
-    if constexpr (G == 32)
+    if constexpr (NINE && G == 32)
       return P.fastg ? gr_svd_u_warp<true>(a, n, w, lane) : gr_svd_u_warp<false>(a, n, w, lane);
     else if constexpr (WARP)
       return P.fastg ? gr_svd_u_grp<G, true>(a, n, w, lane, mask)
@@ -1135,7 +1138,7 @@ __global__ void __launch_bounds__(kBlock, 1) finish_kernel(const __grid_constant
       double chi_new = 0.0;
       if (st == SL_TRIAL) {
         double w[9];
-        const int hits = solve_slot<1, 32>(P, S, s, a, w, nullptr, lane, 0xffffffffu);
+        const int hits = solve_slot<1, 32, true>(P, S, s, a, w, nullptr, lane, 0xffffffffu);
         if (lane == 0) t.svdlim += hits;
         double ptmp[9];
         load9(S.ptmp, W, s, ptmp);
