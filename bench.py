@@ -41,8 +41,13 @@ the same step through the host entry point me_invert_batch with the profiles
 and the results in pinned host memory (host->device copy, inference,
 inversion, device->host copy of the results).
 
-    python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference]
+    python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference] [--details FILE]
     torchrun --nproc-per-node N bench.py --gpus N ...   (one rank per GPU)
+
+The line on stdout is short enough to be kept whole by whoever stores only an
+output's end; everything else that was measured (parity block, histograms,
+rooflines of all kernels, further workloads) goes to --details FILE, or as one
+JSON line to stderr.
 
 With N GPUs every rank inverts its own map (pixels are independent; no
 collective on the data path): scaling is weak, value = all ranks' pixels /
@@ -279,7 +284,42 @@ def parse():
     ap.add_argument("--other-budget-s", type=float, default=480.0,
                     help="wall-time budget of the further workloads; one that would start "
                          "past it is skipped")
+    ap.add_argument("--details", default="",
+                    help="file for everything measured beside the line on stdout "
+                         "(default: stderr)")
     return ap.parse_args()
+
+
+# what the line on stdout keeps of the blocks that go whole to --details
+CONFIG_KEYS = ("workload", "map_pixels", "nl", "num_run", "chisq_criteria", "bounds", "sample",
+               "converged_fraction", "raw_pixels_per_s", "precision", "parallelism", "l2",
+               "converged_sample", "runs_per_pixel", "fallback_rate", "init_ms_per_step")
+ROOFLINE_KEYS = ("bound", "kernel", "achieved", "peak", "unit", "frac", "traffic",
+                 "step_algorithmic_tflops")
+LINE_LIMIT = 2048  # characters
+
+
+def _short(v):
+    if isinstance(v, float):
+        return float(f"{v:.7g}")
+    if isinstance(v, dict):
+        return {k: _short(x) for k, x in v.items()}
+    return [_short(x) for x in v] if isinstance(v, list) else v
+
+
+def stdout_line(full):
+    """The line on stdout of everything measured: the contract's keys, numbers to
+    seven digits, no nested blocks but these."""
+    line = {k: v for k, v in full.items() if k not in ("parity", "other_workloads", "stats")}
+    line["config"] = {k: full["config"][k] for k in CONFIG_KEYS if k in full["config"]}
+    line["roofline"] = {k: full["roofline"][k] for k in ROOFLINE_KEYS if k in full["roofline"]}
+    text = json.dumps(_short(line))
+    for key in reversed(CONFIG_KEYS[7:]):  # (beyond what names the workload)
+        if len(text) <= LINE_LIMIT:
+            break
+        line["config"].pop(key, None)
+        text = json.dumps(_short(line))
+    return text
 
 
 def use_widened(args, workload=None):
@@ -987,9 +1027,8 @@ def main():
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": step_s * 1e3,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
             "dtype": "f32+f64 (MLP bf16)" if args.precision == "FP32" else "f64 (MLP bf16)",
-            "data": "synthetic (seeded draws of the workload's parameter distributions, "
-                    "GPU FP64 synthesis + Gaussian noise; the sample pixels synthesised by "
-                    "the reference core on the host)",
+            "data": "synthetic (seeded draws of the workload's parameter distributions, GPU "
+                    "FP64 synthesis + Gaussian noise; sample pixels synthesised on the host)",
             "config": config,
             "plain_converged_pixels_per_s": plain_conv,
             "learned_vs_plain": learned_vs_plain,
@@ -1030,7 +1069,12 @@ def main():
                            "h2d_ms": e2e["h2d_ms"], "d2h_ms": e2e["d2h_ms"],
                            "steps": e2e["steps"], "warmup": e2e["warmup"],
                            "host_buffers": "page-locked (profiles streamed in chunks)"}
-        print(json.dumps(line), flush=True)
+        if args.details:
+            with open(args.details, "w") as f:
+                json.dump(line, f)
+        else:
+            print(json.dumps(line), file=sys.stderr, flush=True)
+        print(stdout_line(line), flush=True)
     init.close()
     plan.close()
     plain.close()
