@@ -346,6 +346,13 @@ def reference_arm(args):
     if rank != 0:
         return 0
     name = args.workload
+    if cpu_kind(name) != "reference":
+        # the oracle restates the reference; it does not stand in for it here
+        why = ("the reference has no instrument filter"
+               if me_maps.WORKLOADS[name]["ctl"].get("filter", "0") != "0"
+               else "the reference's core is not built here (oracle/_ref, from its sources)")
+        print(json.dumps({"impl": "reference", "unavailable": why}), flush=True)
+        return 0
     widen = use_widened(args)
     cores = host_cores()
     npix = args.npix or me_maps.WORKLOADS[name]["npix"]
