@@ -276,8 +276,8 @@ def parse():
                          "(N = 1 only; 'literal' = the headline map with the literal bounds); "
                          "empty: none")
     ap.add_argument("--svd-registers", type=int, default=-1,
-                    help="me_plan_set_svd_registers for both arms after any autotuning "
-                         "(-1: leave the default / the autotuner's choice)")
+                    help="me_plan_set_svd_registers for both arms (kept for old command "
+                         "lines; it steers nothing any more)")
     ap.add_argument("--kernel-variant", type=int, default=-1,
                     help="me_plan_set_kernel_variant for both arms after any autotuning "
                          "(-1: leave the default / the autotuner's choice)")
@@ -1062,7 +1062,9 @@ def main():
             "cpu_baseline": {"value": out["cpu_value"], "unit": UNIT, "cores": cores,
                              "kind": out["base_kind"],
                              "sample": f"{nb} seeded pixels of the map, "
-                                       f"{cores} processes of the reference core"},
+                                       f"{cores} processes of the "
+                                       + ("reference core" if out["base_kind"] == "reference"
+                                          else "oracle's restatement of it")},
             "parity": parity,
             "other_workloads": others or None,
             "stats": {k: last[k] for k in ("valid", "runs", "iterations", "trials", "accepted",

@@ -214,8 +214,8 @@ int me_plan_svd_registers(const me_plan *plan);
 void me_plan_set_svd_registers(me_plan *plan, int mode);
 /* The LM rounds between two checks of the queue go to the GPU as one CUDA
  * graph, captured once per batch for each lane-group size that runs long
- * enough to repay it (default on; off: one launch per kernel always).  Profiling (me_plan_set_profiling) launches
- * directly. */
+ * enough to repay it (default on; off: one launch per kernel always).
+ * Profiling (me_plan_set_profiling) launches directly. */
 void me_plan_set_graphs(me_plan *plan, int on);
 /* The SVD solves of trials after a rejection run on a second stream beside
  * the Jacobian kernel of the same round (they concern other pixels; default
@@ -319,14 +319,15 @@ int me_faddeeva_weideman(const double *nu, const double *a, long n, double *H, d
  * profiles d_prof [npix][4][nl], ideally of the size and kind the plan will
  * invert) for candidate values of the plan's runtime knobs -- pixels in
  * flight (window), lanes per pixel after the queue drains (max_group), the
- * tail kernel's threshold (tail_slots), lanes per SVD (svd_lanes), the
- * kernel variant (pixels per CTA, grid staging, Faddeeva series reciprocals;
+ * tail kernel's threshold (tail_slots), lanes per SVD (svd_lanes, when a
+ * parameter is fixed), the kernel variant (pixels per CTA, grid staging, Faddeeva series reciprocals;
  * me_plan_set_kernel_variant), the lanes and check interval after the
  * queue drains (me_plan_set_drain), the FP32 Faddeeva evaluation
  * (me_plan_set_faddeeva) and the slot-major profile copy
  * (me_plan_set_slot_profiles) -- one knob at a time, keeping each
- * improvement, and leaves the best setting on the plan.  The carried LM chi^2 is restored afterwards.  out (may be NULL)
- * receives the choice, its time and the number of timed runs. */
+ * improvement, and leaves the best setting on the plan.  The carried LM chi^2
+ * is restored afterwards.  out (may be NULL) receives the choice, its time and
+ * the number of timed runs. */
 typedef struct me_tune_result {
   int window, max_group, tail_slots, svd_lanes;
   double ms;    /* device time of the batch with the chosen setting */
@@ -392,7 +393,8 @@ int me_svd(const double *a, long nmat, int n, double *u, double *w, double *v, i
  * only (the operations on V left out; SVD_solve_mem, Src/LM_FIT.c:400-469,
  * through svdcmp_double, Src/SVD_TEMPLATE.h:84-344), with `lanes` lanes per
  * matrix (1, 2, 4, 8, 16 or 32: one thread, the lane-split rounds, the tail
- * kernel) and the Givens rotations' radius from the reference's pythag and a
+ * kernel; at order 9 always one thread, with the rounding that so many lanes
+ * give) and the Givens rotations' radius from the reference's pythag and a
  * division (fast = 0, FP64 plans) or from one reciprocal square root
  * (fast = 1, FP32 plans).  u and w as me_svd's.  Returns the number of
  * matrices whose QR sweeps hit the 50-sweep limit in *limit_hits (may be
@@ -519,7 +521,11 @@ int me_mlp_save(const me_mlp *mlp, const char *path);
 int me_mlp_load(const char *path, int device, me_mlp **out);
 
 /* Network guess par [npix][9] (the reference's units) for profiles prof
- * [npix][4][nl]: host buffers, or device buffers ordered on `stream`. */
+ * [npix][4][nl]: host buffers, or device buffers ordered on `stream`.  Few
+ * profiles of wide grids (up to 64 of more than 96 wavelengths, 3072 of more
+ * than 192) use the initialiser's batch buffers, which the first such call
+ * allocates; under stream capture, and otherwise, no buffers are needed.  Calls
+ * on several streams are ordered where they share them. */
 int me_mlp_predict(me_mlp *mlp, const double *prof, long npix, double *par);
 int me_mlp_predict_device(me_mlp *mlp, const double *d_prof, long npix, double *d_par,
                           void *stream);

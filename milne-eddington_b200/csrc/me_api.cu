@@ -136,6 +136,7 @@ struct me_plan {
   cudaStream_t stream2 = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   int svd_lanes = 1;  // lanes per matrix of the SVD launches in the full rounds
+  int svd_regs = 0;   // me_plan_set_svd_registers' value, which steers nothing any more
   long long finish_launches = 0;  // tail-kernel launches of the current batch
   // per-kernel device time (me_plan_set_profiling): events recorded around
   // every launch of a batch, read when it ends
@@ -240,7 +241,6 @@ int build_devplan(const me_config *cfg, const double *lambda, int nl, DevPlan &P
   }
   if (P.npar == 0) return fail(ME_ERR_CONFIG, "all nine parameters are fixed");
   // measured defaults on a B200 (the autotuner may choose others)
-  P.svd_regs = 0;
   P.kvar = 0;
   P.faddeeva = cfg->precision == ME_PREC_FP32 ? 1 : 0;
   P.fastg = cfg->precision == ME_PREC_FP32 ? 1 : 0;
@@ -555,7 +555,7 @@ extern "C" int me_plan_poll_trace(const me_plan *p, me_poll_record *out, int cap
 }
 
 extern "C" int me_plan_svd_lanes(const me_plan *p) { return p ? p->svd_lanes : 0; }
-extern "C" int me_plan_svd_registers(const me_plan *p) { return p ? p->P.svd_regs : 0; }
+extern "C" int me_plan_svd_registers(const me_plan *p) { return p ? p->svd_regs : 0; }
 extern "C" int me_plan_kernel_variant(const me_plan *p) { return p ? p->P.kvar : 0; }
 extern "C" void me_plan_set_kernel_variant(me_plan *p, int v) {
   if (p) p->P.kvar = (v >= 0 && v < me::kKernelVariants) ? v : 0;
@@ -579,7 +579,7 @@ extern "C" void me_weideman16(float *coef, float *L) {
   if (L) *L = ME_WEIDEMAN16_L;
 }
 extern "C" void me_plan_set_svd_registers(me_plan *p, int mode) {
-  if (p) p->P.svd_regs = mode <= 0 ? 0 : (mode >= 2 ? 2 : 1);
+  if (p) p->svd_regs = mode <= 0 ? 0 : (mode >= 2 ? 2 : 1);
 }
 extern "C" void me_plan_set_svd_lanes(me_plan *p, int lanes) {
   if (p) p->svd_lanes = lanes >= 8 ? 8 : lanes >= 4 ? 4 : lanes >= 2 ? 2 : 1;
@@ -1624,7 +1624,7 @@ extern "C" int me_plan_autotune(me_plan *p, const double *d_prof, long npix, voi
     out->ms = best;
     out->trials = trials;
     out->kernel_variant = p->P.kvar;
-    out->svd_registers = p->P.svd_regs;
+    out->svd_registers = p->svd_regs;
     out->group_fill = p->group_fill;
     out->drain_poll = p->drain_poll;
     out->faddeeva = p->P.faddeeva;

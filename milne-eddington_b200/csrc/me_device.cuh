@@ -41,9 +41,6 @@ struct DevPlan {
   // variant of the one-thread-per-slot Jacobian and trial kernels (pixels
   // per CTA, grid staging, reciprocal table; me_kernels.h kKernelVariants)
   int kvar;
-  // me_plan_set_svd_registers' value; with all nine parameters free the solves
-  // hold their matrix in registers (svd9_kernel) whatever it says
-  int svd_regs;
   // Faddeeva evaluation of the FP32 syntheses: 0 = the reference's regions
   // and Alg-916, 1 = Weideman's 16-term rational series (FP64 plans: 0)
   int faddeeva;
@@ -1681,8 +1678,8 @@ static __device__ __noinline__ void svd9_cancel(double *t, int rows, double *w, 
 // Every multiply-add is written out, since the results feed an LM that
 // amplifies the last bit: FORM 0 gives gr_svd_u's bits, FORM 1
 // gr_svd_u_grp's, which the compiler fuses differently in the chase's first
-// radius alone.  A NaN matrix, for which no negligible entry is found, is
-// left unrotated.
+// radius alone.  A matrix with NaNs ends too: rv1[0] is zero, so a block's start
+// is always found, and a singular value gets 50 sweeps at most.
 constexpr int kSvd9Words = 9 + 9 + 16;  // doubles of shared memory per thread: w, rv1, cs
 
 // The Householder reduction of A to bidiagonal form (w, rv1); returns anorm.
@@ -1875,7 +1872,7 @@ __device__ __forceinline__ int svd9_sweeps(double (&Q)[R][9], double *w, double 
     }
     // the scalar chain of the sweep; the next step's rv1 and w entries are
     // loaded a step ahead.  With FAST a step takes no branch: one whose radii
-    // leave the exponent window is done again by slow_step.
+    // leave the exponent window is done again below, through radius_slow.
     double gn = rv1[(l + 1) * STR], yn = w[(l + 1) * STR];
     int j = l;
     while (true) {

@@ -6,10 +6,12 @@
 //   outputs: B, cos(theta), sin(2 phi), cos(2 phi), v, Doppler width, a, eta0,
 //            beta, S / I_max, each standardised with the training-set moments.
 //
-// Everything is hand-written here: the data synthesis, BF16 tensor-core GEMMs
-// (mma.sync m16n8k16, FP32 accumulation) with fused bias / GELU epilogues,
-// the backward pass, Adam with FP32 master weights, and the inference that
-// turns a map into per-pixel starting parameters for the LM.  The reference
+// Everything is hand-written here: the data synthesis, the BF16 tensor-core
+// kernels (tcgen05.mma fed by TMA, FP32 accumulators in tensor memory: the whole
+// inference of a map in one, a training step in two) and the separate GEMMs they
+// grew from (tcgen05, or mma.sync m16n8k16 for shapes and settings that ask for
+// it), Adam with FP32 master weights, and the decode that turns the outputs into
+// per-pixel starting parameters for the LM.  The reference
 // has no learned part; the plain LM with its restarts stays the fallback.
 #include <cuda.h>
 #include <cudaTypedefs.h>

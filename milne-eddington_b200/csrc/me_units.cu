@@ -29,7 +29,7 @@ namespace {
 // Measured on a B200, one thread per pixel against this: 262144 profiles of 60
 // wavelengths, FP32, 912 -> 288 us; 10007 FP64 Jacobians of 112 wavelengths 1600
 // -> 533 us; 37 FP32 Jacobians 147 -> 20 us (host call included).  The large FP32
-// map is bound by instruction issue (0.87 per cycle and scheduler).
+// map is bound by instruction issue (0.84 per cycle and scheduler, DRAM at 21 %).
 constexpr int kSynthThreads = 128;
 template <class T>
 constexpr int kSynthPixels = sizeof(T) == sizeof(float) ? 32 : 16;  // most per block

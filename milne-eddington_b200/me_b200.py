@@ -511,8 +511,8 @@ class Plan:
 
     @property
     def svd_registers(self) -> int:
-        """SVD solves with the 9x9 matrix in registers (all nine parameters free):
-        0 shared memory, 1 registers in the full rounds, 2 also after the drain."""
+        """Kept for programs that set it: the solves with all nine parameters free
+        hold their matrix in registers whatever it says."""
         return lib().me_plan_svd_registers(self._h)
 
     @svd_registers.setter
