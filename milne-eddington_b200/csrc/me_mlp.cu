@@ -744,9 +744,9 @@ __global__ void decode_kernel(const float *Y, long long n, int ld, const float *
 // The values are those of map_features_kernel, umma_gemm_kernel and
 // decode_kernel, which did this in six launches with every layer's activations
 // through memory.  Profiles of 60 wavelengths, there and here, us:
-//   1: 46, 45;  1,000: 53, 47;  18,900: 90, 50;  37,889: 162, 95;  300,007: 921, 493
-// and of 112: 1: 52, 51;  18,900: 106, 56;  75,000: 313, 163.  Few profiles of
-// more features go through the six launches all the same: see predict_separately.
+//   1: 46, 45;  1,000: 52, 47;  18,900: 89, 50;  37,889: 162, 96;  300,007: 920, 496
+// and of 112: 18,900: 102, 55;  75,000: 311, 164.  Few profiles of more features
+// go through the six launches all the same: see predict_separately.
 // Waits are bounded.  The first to run out writes a code to *err (1: weights, 2: a
 // free stage, 3: the accumulator) and raises the CTA's stop flag, at which all
 // other waits end too.  The named barriers have no limit: every warp passes each
