@@ -165,11 +165,6 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
                : "memory");
 }
 
-// one plain arrival on `bar`
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-
 // makes this thread's shared-memory writes visible to the tensor cores
 __device__ __forceinline__ void fence_smem_to_async() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
